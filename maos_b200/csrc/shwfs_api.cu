@@ -983,24 +983,23 @@ static int l2_bytes(shwfs_ctx* ctx) {
 	return v;
 }
 
-// The open-loop trace kernel for 16x16 or 32x32 pupils and 1-8 layers (their
-// tables stay below the 48 KB default of dynamic shared memory).
-using GeomKernel = void (*)(const GeomParams, int, int, int);
-template <int NOPD>
-static GeomKernel geom_pick_n(int nl) {
-	switch (nl) {
-	case 1: return geom_kernel<false, NOPD, 1>;
-	case 2: return geom_kernel<false, NOPD, 2>;
-	case 3: return geom_kernel<false, NOPD, 3>;
-	case 4: return geom_kernel<false, NOPD, 4>;
-	case 5: return geom_kernel<false, NOPD, 5>;
-	case 6: return geom_kernel<false, NOPD, 6>;
-	case 7: return geom_kernel<false, NOPD, 7>;
-	case 8: return geom_kernel<false, NOPD, 8>;
-	default: return geom_kernel<false, NOPD, 0>;
-	}
+// 16x16 and 32x32 pupils (geom_rows_kernel)
+template <bool EXTRA, int NOPD, int ROWS>
+static void geom_rows_launch(const GeomParams& gp, int nitem, cudaStream_t st) {
+	constexpr int PPB = geom_rows_pupils(NOPD, ROWS);
+	const size_t smem = (size_t)PPB * gp.nlayer * geom_rows_bytes(NOPD);
+	geom_rows_kernel<EXTRA, NOPD, ROWS>
+		<<<(nitem + PPB - 1) / PPB, 32 * geom_rows_warps(NOPD, ROWS) * PPB, smem, st>>>(gp, nitem);
 }
-static GeomKernel geom_pick(int nopd, int nl) { return nopd == 16 ? geom_pick_n<16>(nl) : geom_pick_n<32>(nl); }
+// Launches of fewer points per SM than this run the two-row form: a launch of
+// 2048 points per SM is eight warps of the eight-row form, too few to hide its
+// chain of layers.
+constexpr long GEOM_SMALL_POINTS = 2048;
+template <bool EXTRA>
+static void geom_rows_pick(const GeomParams& gp, int nopd, int nitem, bool small, cudaStream_t st) {
+	if (nopd == 16) (small ? geom_rows_launch<EXTRA, 16, 2> : geom_rows_launch<EXTRA, 16, 8>)(gp, nitem, st);
+	else (small ? geom_rows_launch<EXTRA, 32, 2> : geom_rows_launch<EXTRA, 32, 8>)(gp, nitem, st);
+}
 
 // split: when the launch's screens exceed L2, the pupils of the largest size
 // are traced interleaved (each screen row their footprints share is fetched
@@ -1065,16 +1064,22 @@ static int launch_geom_wfs(shwfs_ctx* ctx, GeomParams& gp, bool split) {
 		const int np = nopd * nopd;
 		const int bd = std::min(256, std::max(32, ((np + GEOM_PTS - 1) / GEOM_PTS + 31) / 32 * 32));
 		int bps = (np + GEOM_PTS * bd - 1) / (GEOM_PTS * bd);  // blocks per subaperture
-		const bool fixed = !extra && (nopd == 16 || nopd == 32) && gp.nlayer <= 8;
+		bool rows = nopd == 16 || nopd == 32;  // whose tables hold element offsets of 30 bits
+		for (int l = 0; l < gp.nlayer; l++) rows = rows && (long)gp.nx[l] * gp.ny[l] < (1L << 30);
 		gp.ppt = GEOM_PTS;
-		if (!fixed && (long)nblk * bps < sm_count(ctx)) {  // a few pupils: a point per thread, more blocks
+		if (!rows && (long)nblk * bps < sm_count(ctx)) {  // a few pupils: a point per thread, more blocks
 			gp.ppt = 1;
 			bps = (np + bd - 1) / bd;
 		}
-		if (extra) geom_kernel<true><<<(unsigned)nblk * bps, bd, smem, ctx->stream>>>(gp, nopd, nitem, bps);
-		else if (fixed)  // pupil side and layer count fixed at compile time
-			geom_pick(nopd, gp.nlayer)<<<(unsigned)nblk * bps, bd, smem, ctx->stream>>>(gp, nopd, nitem, bps);
-		else geom_kernel<false><<<(unsigned)nblk * bps, bd, smem, ctx->stream>>>(gp, nopd, nitem, bps);
+		if (rows) {
+			const bool small = (long)nitem * np < GEOM_SMALL_POINTS * sm_count(ctx);
+			if (extra) geom_rows_pick<true>(gp, nopd, nitem, small, ctx->stream);
+			else geom_rows_pick<false>(gp, nopd, nitem, small, ctx->stream);
+		} else if (extra) {
+			geom_kernel<true><<<(unsigned)nblk * bps, bd, smem, ctx->stream>>>(gp, nopd, nitem, bps);
+		} else {
+			geom_kernel<false><<<(unsigned)nblk * bps, bd, smem, ctx->stream>>>(gp, nopd, nitem, bps);
+		}
 	}
 	CK(cudaGetLastError());
 	return 0;

@@ -16,6 +16,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <type_traits>
 #include "fft_reg.cuh"
 
 namespace shwfs {
@@ -409,13 +410,9 @@ __device__ __forceinline__ float geom_bilerp(float al, float m00, float m10, flo
 
 // EXTRA: the launch has mirror grids, NCPA surfaces or polynomial terms (a
 // closed-loop frame); the open-loop launch compiles without their code.
-// NOPD: the pupil side at compile time (0: the nopd argument; 16 launches
-// 64-thread blocks, 32 256-thread blocks); NL: the layer count at compile time
-// (0: P.nlayer).
-template <bool EXTRA, int NOPD = 0, int NL = 0>
-__global__ void __launch_bounds__(NOPD == 16 ? 64 : 256, NOPD == 16 ? 32 : NOPD == 32 ? 8 : 1)
-	geom_kernel(const __grid_constant__ GeomParams P, int nopd_arg, int nitem, int bps) {
-	const int nopd = NOPD ? NOPD : nopd_arg;
+// 16x16 and 32x32 pupils run geom_rows_kernel below instead.
+template <bool EXTRA>
+__global__ void __launch_bounds__(256) geom_kernel(const __grid_constant__ GeomParams P, int nopd, int nitem, int bps) {
 	extern __shared__ int4 s_tab[];
 	const int item = blockIdx.x / bps, part = blockIdx.x - item * bps;
 	if (item >= nitem) return;
@@ -428,8 +425,7 @@ __global__ void __launch_bounds__(NOPD == 16 ? 64 : 256, NOPD == 16 ? 32 : NOPD 
 		isa = item - P.e[ie].item0;
 	}
 	const GeomEntry& E = P.e[ie];
-	const int tid = threadIdx.x, nl = NL ? NL : P.nlayer;
-	const int bdim = NOPD == 16 ? 64 : NOPD == 32 ? 256 : (int)blockDim.x;
+	const int tid = threadIdx.x, nl = P.nlayer, bdim = blockDim.x;
 	// the footprint origin of each (layer, axis) once, in FP64; then the
 	// entries of the nopd points of each line from it in FP32
 	__shared__ int s_j0[2 * SHWFS_MAX_LAYERS];
@@ -461,7 +457,7 @@ __global__ void __launch_bounds__(NOPD == 16 ? 64 : 256, NOPD == 16 ? 32 : NOPD 
 	// up to GEOM_PTS points per thread, layers outermost so that the gathers of the points are in flight
 	// together; every point still sums its layers in order
 	const int bd = bdim;
-	const int pts = NOPD || P.ppt <= 0 || P.ppt > GEOM_PTS ? GEOM_PTS : P.ppt;
+	const int pts = P.ppt <= 0 || P.ppt > GEOM_PTS ? GEOM_PTS : P.ppt;
 	const int np = nopd * nopd, p0 = pts * bd * part, p1 = min(np, p0 + pts * bd);
 	float acc[GEOM_PTS];
 	int ixu[GEOM_PTS], iyu[GEOM_PTS];
@@ -473,20 +469,14 @@ __global__ void __launch_bounds__(NOPD == 16 ? 64 : 256, NOPD == 16 ? 32 : NOPD 
 		iyu[u] = ip / nopd;
 	}
 	const int nwrap = EXTRA ? nl - P.nmirror : nl;
-	// 16x16 and 32x32 pupils: a thread's points fill whole rows of one column
-	// (64 or 256 threads, four rows apart), so they share the column entry and
-	// need no bounds test
-	constexpr bool ONECOL = NOPD == 16 || NOPD == 32;
-#pragma unroll
 	for (int l = 0; l < nwrap; l++) {
 		if (!((E.use >> l) & 1u)) continue;
 		const float* __restrict__ sc = P.screen[l];
 		const float al = P.alpha[l];
-		const int4 tx0 = s_tab[l * 2 * nopd + ixu[0]];
 #pragma unroll
 		for (int u = 0; u < GEOM_PTS; u++) {
-			if (ONECOL || p0 + tid + bd * u < p1) {
-				const int4 tx = ONECOL ? tx0 : s_tab[l * 2 * nopd + ixu[u]], ty = s_tab[l * 2 * nopd + nopd + iyu[u]];
+			if (p0 + tid + bd * u < p1) {
+				const int4 tx = s_tab[l * 2 * nopd + ixu[u]], ty = s_tab[l * 2 * nopd + nopd + iyu[u]];
 				const float m00 = __ldg(sc + (ty.x + tx.x)), m10 = __ldg(sc + (ty.x + tx.y));
 				const float m01 = __ldg(sc + (ty.y + tx.x)), m11 = __ldg(sc + (ty.y + tx.y));
 				acc[u] = geom_bilerp(al, m00, m10, m01, m11, __int_as_float(tx.z), __int_as_float(ty.z), acc[u]);
@@ -520,6 +510,191 @@ __global__ void __launch_bounds__(NOPD == 16 ? 64 : 256, NOPD == 16 ? 32 : NOPD 
 #pragma unroll
 	for (int u = 0; u < GEOM_PTS; u++)
 		if (p0 + tid + bd * u < p1) E.opd[(size_t)isa * np + p0 + tid + bd * u] = acc[u];
+}
+
+// ---- 16x16 and 32x32 pupils: geom_rows_kernel ----
+// The gathers of geom_kernel are bound by L1 wavefronts (a half-row of 16
+// points costs one or two of them per load, whatever it reuses).  Here a lane
+// owns one column of the pupil and walks ROWS consecutive rows of it: the lower
+// screen row of a point is the upper row of the next point, or the same row
+// again, wherever the pupil is sampled no coarser than the screen, so the
+// interpolation along x of a screen row is formed once and kept in registers
+// and a point costs two gathers or none instead of four.  The row entries say
+// which; a layer with a row that skips a screen row (pupil sampling coarser
+// than the screen) gathers both rows of every point.  One warp covers the two
+// column halves of a 16x16 pupil or the 32 columns of a 32x32 one; the lanes
+// build a layer's line entries together.  The OPD is that of geom_kernel to
+// the bit.  Measured against four gathers a point (7 layers, 6 WFS of 2820
+// pupils): 16x16 63 -> 43 us, with two mirrors and focus 117 -> 55 us; 32x32
+// from 4096^2 screens 201 -> 124 us; three science directions 136 -> 85 us.
+// What bounds it now: L1 wavefronts (7.9 M of a 16x16 launch, 28 us) and
+// issue (26 M warp instructions, 24 us) beside each other at 32 warps per SM;
+// 24 or 40 warps per SM (80 or 48 registers a thread) measured 3 % and 60 %
+// slower.
+// ROWS: 8 where the launch fills the chip, 2 (four times the warps, shorter
+// chains) where it does not; the choice is geom_rows_pick's.
+__host__ __device__ constexpr int geom_rows_warps(int nopd, int rows) { return nopd * nopd / (32 * rows); }
+__host__ __device__ constexpr int geom_rows_pupils(int nopd, int rows) {  // pupils per block
+	return geom_rows_warps(nopd, rows) == 1 ? 2 : 1;
+}
+__host__ __device__ constexpr int geom_rows_min_blocks(int nopd, int rows) {  // 32 warps per SM: 64 registers a thread
+	return 32 / (geom_rows_warps(nopd, rows) * geom_rows_pupils(nopd, rows));
+}
+// shared memory of one pupil and layer: the column entries (first and second
+// screen column, weight, valid), the row entries (offset of the second screen
+// row, or -1 where both rows are those of the point before; weight) and both
+// rows' offsets (the first doubled, with valid in its low bit)
+__host__ __device__ constexpr int geom_rows_bytes(int nopd) { return nopd * (16 + 8 + 8); }
+
+// the two steps of geom_bilerp
+__device__ __forceinline__ float geom_xlerp(float m0, float m1, float w) { return fmaf(m1 - m0, w, m0); }
+__device__ __forceinline__ float geom_ylerp(float lo, float hi, float w) { return fmaf(lo, 1.f - w, hi * w); }
+// m0, m1 = p[0], p[1] where off >= 0, undefined else: predicated, so that the
+// loads of all rows of a lane are in flight together
+__device__ __forceinline__ void geom_pair_if(const float* p, int off, float& m0, float& m1) {
+	asm("{\n\t.reg .pred p;\n\tsetp.ge.s32 p, %3, 0;\n\t@p ld.global.nc.f32 %0, [%2];\n\t@p ld.global.nc.f32 %1, [%2+4];\n\t}"
+		: "=f"(m0), "=f"(m1)
+		: "l"(p), "r"(off));
+}
+
+template <bool EXTRA, int NOPD, int ROWS>
+__global__ void __launch_bounds__(32 * geom_rows_warps(NOPD, ROWS) * geom_rows_pupils(NOPD, ROWS),
+	geom_rows_min_blocks(NOPD, ROWS)) geom_rows_kernel(const __grid_constant__ GeomParams P, int nitem) {
+	constexpr int WPS = geom_rows_warps(NOPD, ROWS), PPB = geom_rows_pupils(NOPD, ROWS);
+	constexpr int NP = NOPD * NOPD;
+	extern __shared__ int4 s_tab[];
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const int sub = warp / WPS, wsub = warp % WPS;  // pupil of the block, warp of the pupil
+	const int nl = P.nlayer, nwrap = EXTRA ? nl - P.nmirror : nl;
+	auto pupil = [&](int item, int& ie, int& isa) {
+		ie = 0;
+		if (P.interleave) {
+			ie = item % P.nentry;
+			isa = item / P.nentry;
+		} else {
+			while (ie + 1 < P.nentry && item >= P.e[ie + 1].item0) ie++;
+			isa = item - P.e[ie].item0;
+		}
+	};
+	char* tab = reinterpret_cast<char*>(s_tab) + sub * nl * geom_rows_bytes(NOPD);
+	__shared__ int4 s_org[PPB][2 * SHWFS_MAX_LAYERS];  // per (layer, axis): first index, fraction, step, points
+	__shared__ unsigned s_slow[PPB][SHWFS_MAX_LAYERS];  // not 0: a row skips a screen row, or a column wraps
+	// the FP64 footprint origins of the block's pupils, a thread each
+	for (int k = threadIdx.x; k < PPB * 2 * nl; k += 32 * WPS * PPB) {
+		const int q = k / (2 * nl), r = k - q * 2 * nl, l = r >> 1;
+		if (blockIdx.x * PPB + q >= nitem) break;
+		int je, jsa, j0;
+		float f0;
+		pupil(blockIdx.x * PPB + q, je, jsa);
+		geom_origin<EXTRA>(P, P.e[je], jsa, l, r & 1, j0, f0);
+		s_org[q][r] = make_int4(j0, __float_as_int(f0), __float_as_int((float)(P.e[je].dx * P.e[je].sx[l])),
+			r & 1 ? P.ny[l] : P.nx[l]);
+	}
+	__syncthreads();
+	if (PPB > 1 && blockIdx.x * PPB + sub >= nitem) return;  // one warp per pupil: no block barrier below
+	int ie, isa;
+	pupil(blockIdx.x * PPB + sub, ie, isa);
+	const GeomEntry& E = P.e[ie];
+	for (int l = wsub; l < nl; l += WPS) {
+		int4* tx = reinterpret_cast<int4*>(tab + l * geom_rows_bytes(NOPD));
+		int2* ty = reinterpret_cast<int2*>(tx + NOPD);
+		int2* ty0 = ty + NOPD;
+		unsigned slow = 0;
+#pragma unroll
+		for (int t = 2 * NOPD / 32 - 1; t >= 0; t--) {
+			const bool isy = NOPD == 16 ? lane >= 16 : t == 1;
+			const int i = NOPD == 16 ? lane & 15 : lane;
+			const int4 o = s_org[sub][2 * l + isy];
+			int j, j1, valid = 1;
+			float w;
+			if (!EXTRA || l < nwrap) geom_point(o.x, __int_as_float(o.y), i, __int_as_float(o.z), o.w, j, j1, w);
+			else geom_point_clip(o.x, __int_as_float(o.y), i, __int_as_float(o.z), o.w, j, j1, w, valid);
+			// the row's relation to the row before it in the same lane's walk
+			const int jp = __shfl_up_sync(0xffffffffu, j, 1), jp1 = __shfl_up_sync(0xffffffffu, j1, 1);
+			const bool first = i % ROWS == 0, same = j == jp && j1 == jp1;
+			slow |= __ballot_sync(0xffffffffu, isy ? !first && !same && j != jp1 : j1 != j + 1);
+			if (isy) {
+				const int m = P.nx[l];
+				ty[i] = make_int2(!first && same ? -1 : j1 * m, __float_as_int(w));
+				ty0[i] = make_int2(2 * (j * m) | valid, j1 * m);
+			} else {
+				tx[i] = make_int4(j, j1, __float_as_int(w), valid);
+			}
+		}
+		if (lane == 0) s_slow[sub][l] = slow;
+	}
+	if (WPS == 1) __syncwarp();
+	else __syncthreads();
+	const int ix = NOPD == 16 ? lane & 15 : lane;
+	const int iy0 = NOPD == 16 ? (wsub * 2 + (lane >> 4)) * ROWS : wsub * ROWS;
+	float acc[ROWS];
+#pragma unroll
+	for (int u = 0; u < ROWS; u++) acc[u] = 0.f;
+	auto layer = [&](int l, auto mirror) {  // one layer, or one mirror grid
+		constexpr bool MIRROR = decltype(mirror)::value;
+		const float al = P.alpha[l];
+		const char* t = tab + l * geom_rows_bytes(NOPD);
+		const int4 tx = reinterpret_cast<const int4*>(t)[ix];
+		const int4* ty = reinterpret_cast<const int4*>(t + NOPD * 16 + iy0 * 8);  // two rows each
+		const int2* ty0 = reinterpret_cast<const int2*>(t + NOPD * 24) + iy0;
+		const float* sc = P.screen[l];
+		const float wx = __int_as_float(tx.z);
+		// mirror grids: NaN marks grid points outside the mirror (add_valid, math/numtype.h:40)
+		auto add = [&](int u, float v) {
+			if (!MIRROR || ((tx.w & ty0[u].x & 1) && !isnan(v))) acc[u] = fmaf(al, v, acc[u]);
+		};
+		if (s_slow[sub][l] == 0) {
+			int off[ROWS];
+			float w[ROWS], n0[ROWS], n1[ROWS];
+#pragma unroll
+			for (int u = 0; u < ROWS; u += 2) {
+				const int4 e = ty[u / 2];
+				off[u] = e.x;
+				w[u] = __int_as_float(e.y);
+				off[u + 1] = e.z;
+				w[u + 1] = __int_as_float(e.w);
+			}
+			const float* p = sc + ((ty0[0].x >> 1) + tx.x);
+			const float m0 = __ldg(p), m1 = __ldg(p + 1);
+#pragma unroll
+			for (int u = 0; u < ROWS; u++) geom_pair_if(sc + (off[u] + tx.x), off[u], n0[u], n1[u]);
+			float lo = geom_xlerp(m0, m1, wx), hi = 0.f;
+#pragma unroll
+			for (int u = 0; u < ROWS; u++) {
+				const float x = geom_xlerp(n0[u], n1[u], wx);
+				if (u > 0) lo = off[u] >= 0 ? hi : lo;
+				hi = u == 0 || off[u] >= 0 ? x : hi;
+				add(u, geom_ylerp(lo, hi, w[u]));
+			}
+		} else {
+#pragma unroll
+			for (int u = 0; u < ROWS; u++) {
+				const int o0 = ty0[u].x >> 1, o1 = ty0[u].y;
+				const float lo = geom_xlerp(__ldg(sc + (o0 + tx.x)), __ldg(sc + (o0 + tx.y)), wx);
+				const float hi = geom_xlerp(__ldg(sc + (o1 + tx.x)), __ldg(sc + (o1 + tx.y)), wx);
+				add(u, geom_ylerp(lo, hi, reinterpret_cast<const float*>(ty)[2 * u + 1]));
+			}
+		}
+	};
+	for (int l = 0; l < nwrap; l++)
+		if ((E.use >> l) & 1u) layer(l, std::false_type());
+	for (int l = nwrap; EXTRA && l < nl; l++)
+		if ((E.use >> l) & 1u) layer(l, std::true_type());
+	if (EXTRA && E.opdadd) {
+#pragma unroll
+		for (int u = 0; u < ROWS; u++) acc[u] += E.opdadd[(size_t)isa * NP + (iy0 + u) * NOPD + ix];
+	}
+	if (EXTRA && E.has_poly) {  // geom_extra's polynomial, its x and y parts apart
+		const double x = E.origx[isa] + ix * E.dx, px = E.poly[0] + x * (E.poly[1] + E.poly[3] * x);
+#pragma unroll
+		for (int u = 0; u < ROWS; u++) {
+			const double y = E.origy[isa] + (iy0 + u) * E.dx;
+			acc[u] += (float)(px + y * (E.poly[2] + E.poly[3] * y));
+		}
+	}
+	float* o = E.opd + (size_t)isa * NP + iy0 * NOPD + ix;
+#pragma unroll
+	for (int u = 0; u < ROWS; u++) o[u * NOPD] = acc[u];
 }
 
 // LGS uplink: ray trace of each LLT pupil (one block of 256 threads per
