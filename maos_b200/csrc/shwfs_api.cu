@@ -1928,26 +1928,66 @@ int shwfs_addnoise_dev(shwfs_ctx* ctx, float* ints, long n, const float* bkgrnd2
 	return 0;
 }
 
-// Geometric gradients of one WFS from its OPD (one warp per subaperture):
-// z-tilt, or G-tilt with the WFS's GS0.
-static int launch_geom_grad(shwfs_ctx* ctx, WfsState& w, const float* opd, float* grad, bool noisy, int isim) {
-	PowfsState& p = ctx->powfs[w.d.ipowfs];
+// z-tilt gradients of WFS of powfs p from their OPDs, a launch per
+// SHWFS_MAX_ENTRIES of them.  One launch serves the six WFS of the 30 m LGS
+// system: six launches of 353 blocks each spent most of their time on the
+// gaps between them and on their tails.
+struct ZtiltJob {
+	const WfsState* w;
+	const float* opd;
+	float* grad;
+	bool noisy;
+};
+static int launch_ztilt(shwfs_ctx* ctx, const PowfsState& p, const std::vector<ZtiltJob>& jobs, int isim) {
 	const int nsa = p.d.nsa;
-	const float* nea = noisy ? w.neasim.p : nullptr;
-	const uint32_t wid = (uint32_t)(&w - ctx->wfs.data());
-	if (p.d.gradtype == SHWFS_GRAD_GTILT) {
-		const size_t m = p.namp > 1 ? (size_t)w.wfsind : 0;
-		if (m >= p.gs0_ptr.size() || !p.gs0_ptr[m].p) return fail(ctx, SHWFS_ESTATE, "G-tilt operator GS0 not set");
+	for (size_t k0 = 0; k0 < jobs.size(); k0 += SHWFS_MAX_ENTRIES) {
+		ZtiltParams Z;
+		memset(&Z, 0, sizeof(Z));
+		const int n = (int)std::min((size_t)SHWFS_MAX_ENTRIES, jobs.size() - k0);
+		for (int k = 0; k < n; k++) {
+			const ZtiltJob& j = jobs[k0 + k];
+			Z.w[k].opd = j.opd;
+			Z.w[k].amp = p.amp.p + (p.namp > 1 ? (size_t)j.w->wfsind * nsa * p.d.nopd * p.d.nopd : 0);
+			Z.w[k].nea = j.noisy ? j.w->neasim.p : nullptr;
+			Z.w[k].grad = j.grad;
+			Z.w[k].seed = j.w->seed;
+			Z.w[k].wfs_id = (uint32_t)(j.w - ctx->wfs.data());
+		}
 		StageMark mk(ctx, SHWFS_STAGE_POST);
-		gtilt_kernel<<<(nsa + 7) / 8, 256, 0, ctx->stream>>>(p.gs0_ptr[m].p, p.gs0_col[m].p, p.gs0_val[m].p, nsa, opd,
-			grad, nea, w.seed, wid, (uint32_t)isim);
-	} else {
-		const float* amp = p.amp.p + (p.namp > 1 ? (size_t)w.wfsind * nsa * p.d.nopd * p.d.nopd : 0);
-		StageMark mk(ctx, SHWFS_STAGE_POST);
-		ztilt_kernel<<<(nsa + 7) / 8, 256, 0, ctx->stream>>>(opd, amp, p.origx.p, p.origy.p, nsa, p.d.nopd, p.d.dx,
-			grad, nea, w.seed, wid, (uint32_t)isim);
+		ztilt_kernel<<<dim3((nsa + 7) / 8, n), 256, 0, ctx->stream>>>(Z, p.origx.p, p.origy.p, nsa, p.d.nopd, p.d.dx,
+			(uint32_t)isim);
+		CK(cudaGetLastError());
 	}
+	return 0;
+}
+
+// G-tilt gradients of one WFS from its OPD with its GS0 (one warp per subaperture).
+static int launch_gtilt(shwfs_ctx* ctx, const WfsState& w, const float* opd, float* grad, bool noisy, int isim) {
+	const PowfsState& p = ctx->powfs[w.d.ipowfs];
+	const int nsa = p.d.nsa;
+	const size_t m = p.namp > 1 ? (size_t)w.wfsind : 0;
+	if (m >= p.gs0_ptr.size() || !p.gs0_ptr[m].p) return fail(ctx, SHWFS_ESTATE, "G-tilt operator GS0 not set");
+	StageMark mk(ctx, SHWFS_STAGE_POST);
+	gtilt_kernel<<<(nsa + 7) / 8, 256, 0, ctx->stream>>>(p.gs0_ptr[m].p, p.gs0_col[m].p, p.gs0_val[m].p, nsa, opd,
+		grad, noisy ? w.neasim.p : nullptr, w.seed, (uint32_t)(&w - ctx->wfs.data()), (uint32_t)isim);
 	CK(cudaGetLastError());
+	return 0;
+}
+
+// Geometric gradients of the WFS wl of a powfs from their traced OPDs.
+static int launch_geom_grad(shwfs_ctx* ctx, const PowfsState& p, const std::vector<int>& wl, int isim) {
+	if (p.d.gradtype == SHWFS_GRAD_ZTILT) {
+		std::vector<ZtiltJob> jobs;
+		for (int i : wl) {
+			const WfsState& w = ctx->wfs[i];
+			jobs.push_back({&w, w.opd.p, w.grad.p, w.d.noisy && w.neasim.p});
+		}
+		return launch_ztilt(ctx, p, jobs, isim);
+	}
+	for (int i : wl) {
+		const WfsState& w = ctx->wfs[i];
+		if (int r = launch_gtilt(ctx, w, w.opd.p, w.grad.p, w.d.noisy && w.neasim.p, isim)) return r;
+	}
 	return 0;
 }
 
@@ -1966,11 +2006,7 @@ static int frame_powfs(shwfs_ctx* ctx, int ip, const std::vector<int>& wl, int i
 			}
 			if ((r = launch_geom(ctx, gp))) return r;
 		}
-		for (int i : wl) {
-			WfsState& w = ctx->wfs[i];
-			if ((r = launch_geom_grad(ctx, w, w.opd.p, w.grad.p, w.d.noisy && w.neasim.p, isim))) return r;
-		}
-		return 0;
+		return launch_geom_grad(ctx, p, wl, isim);
 	}
 	if ((r = trace_powfs(ctx, ip, wl, isim))) return r;
 	// (b)-(e)
@@ -2622,12 +2658,7 @@ int shwfs_grad_ztilt_dev(shwfs_ctx* ctx, int iwfs, const float* opd, float* grad
 	const PowfsState& p = ctx->powfs[w->d.ipowfs];
 	if (!p.amp.p || !p.origx.p) return fail(ctx, SHWFS_ESTATE, "powfs geometry not set");
 	// the z-tilt fit on any powfs's geometry
-	const int nsa = p.d.nsa;
-	const float* amp = p.amp.p + (p.namp > 1 ? (size_t)w->wfsind * nsa * p.d.nopd * p.d.nopd : 0);
-	ztilt_kernel<<<(nsa + 7) / 8, 256, 0, ctx->stream>>>(opd, amp, p.origx.p, p.origy.p, nsa, p.d.nopd, p.d.dx, grad,
-		nullptr, 0, 0, 0);
-	CK(cudaGetLastError());
-	return 0;
+	return launch_ztilt(ctx, p, {{w, opd, grad, false}}, 0);
 }
 
 int shwfs_grad_gtilt_dev(shwfs_ctx* ctx, int iwfs, const float* opd, float* grad) {
@@ -2637,7 +2668,7 @@ int shwfs_grad_gtilt_dev(shwfs_ctx* ctx, int iwfs, const float* opd, float* grad
 	if (r) return r;
 	if (ctx->powfs[w->d.ipowfs].d.gradtype != SHWFS_GRAD_GTILT)
 		return fail(ctx, SHWFS_EINVAL, "grad_gtilt: the powfs is not a G-tilt sensor");
-	return launch_geom_grad(ctx, *w, opd, grad, false, 0);
+	return launch_gtilt(ctx, *w, opd, grad, false, 0);
 }
 
 int shwfs_powfs_set_gs0(shwfs_ctx* ctx, int ipowfs, int iamp, long nrow, long ncol, const int* pp, const int* pi,

@@ -1247,9 +1247,21 @@ __device__ __forceinline__ void geom_noise(float& gx, float& gy, int isa, int ns
 // g = [(b0, b1, b2) . imcc(:, 1), (b0, b1, b2) . imcc(:, 2)], b = (sum a o,
 // sum a o x, sum a o y), imcc = inv(sum a [1 x y]'[1 x y]), x = origx + ix dx.
 // One warp per subaperture, FP64 sums; with nea, geom_noise is added.
-__global__ void ztilt_kernel(const float* __restrict__ opd, const float* __restrict__ amp,
-	const double* __restrict__ origx, const double* __restrict__ origy, int nsa, int nopd, double dx,
-	float* __restrict__ grad, const float* __restrict__ nea, uint64_t seed, uint32_t wfs_id, uint32_t frame) {
+// blockIdx.y is the WFS: one launch serves every WFS of a powfs.
+struct ZtiltWfs {
+	const float *opd, *amp, *nea;
+	float* grad;
+	uint64_t seed;
+	uint32_t wfs_id;
+};
+struct ZtiltParams {
+	ZtiltWfs w[SHWFS_MAX_ENTRIES];
+};
+__global__ void __launch_bounds__(256) ztilt_kernel(const __grid_constant__ ZtiltParams Z,
+	const double* __restrict__ origx, const double* __restrict__ origy, int nsa, int nopd, double dx, uint32_t frame) {
+	const ZtiltWfs& W = Z.w[blockIdx.y];
+	const float* __restrict__ opd = W.opd;
+	const float* __restrict__ amp = W.amp;
 	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 	const int isa = blockIdx.x * (blockDim.x >> 5) + warp;
 	if (isa >= nsa) return;
@@ -1284,9 +1296,9 @@ __global__ void ztilt_kernel(const float* __restrict__ opd, const float* __restr
 			gx = (float)((m[6] * c01 + m[7] * c11 + m[8] * c12) / det);
 			gy = (float)((m[6] * c02 + m[7] * c12 + m[8] * c22) / det);
 		}
-		if (nea) geom_noise(gx, gy, isa, nsa, nea, seed, wfs_id, frame);
-		grad[isa] = gx;
-		grad[isa + nsa] = gy;
+		if (W.nea) geom_noise(gx, gy, isa, nsa, W.nea, W.seed, W.wfs_id, frame);
+		W.grad[isa] = gx;
+		W.grad[isa + nsa] = gy;
 	}
 }
 
