@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(GEN_PIX_THREADS) gen_pixels_block_kernel(Powfs
 }
 
 // ---------------------------------------------------------------------------
-// n_f = n_w = 64 fused per image: one block of 256 threads holds the 64x64
+// n_f = n_w = 64 fused per image: one block of 128 threads holds the 64x64
 // image in shared memory; every 64-point line transform is 8 x 8: n = 8 n1 +
 // n2, k = k1 + 8 k2, X[k] = sum_n2 w64^(n2 k1) w8^(n2 k2) sum_n1 x[n] w8^(n1 k1),
 // with the 8-point transforms in registers, so each line costs two passes
@@ -391,16 +391,10 @@ constexpr int N64_LS = 65;  // line stride of the shared image (float2): row, co
 
 __device__ __forceinline__ int digrev8(int k) { return ((k & 7) << 3) | (k >> 3); }
 
-// 8-point DFT in registers, natural order in and out; dir -1 forward, +1 inverse
-__device__ __forceinline__ void dft8(float2 (&a)[8], float dir) {
+// 8-point DFT in registers, natural order in and out; dir -1 forward, +1
+// inverse.  dft8_tail: what follows the radix-2 stage on the pairs (j, j+4).
+__device__ __forceinline__ void dft8_tail(float2 (&b)[8], float2 (&a)[8], float dir) {
 	const float h = 0.70710678118654752f;
-	// radix-2 stage on pairs (j, j+4)
-	float2 b[8];
-#pragma unroll
-	for (int j = 0; j < 4; j++) {
-		b[j] = make_float2(a[j].x + a[j + 4].x, a[j].y + a[j + 4].y);
-		b[j + 4] = make_float2(a[j].x - a[j + 4].x, a[j].y - a[j + 4].y);
-	}
 	// twiddles w8^j on b[4..7]: w8 = exp(dir i pi/4)
 	{
 		float2 t = b[5];
@@ -424,196 +418,340 @@ __device__ __forceinline__ void dft8(float2 (&a)[8], float dir) {
 	}
 }
 
-// One 64-point transform of NLINES lines (nlines when NLINES is 0) of the
-// 64 x N64_LS shared image: rows (line L at s + (line0 + L) * N64_LS, element
-// j at + j) or columns (COLS: line L at s + line0 + L, element j at + j *
-// N64_LS), in form F (DIGREV_IN false) or G (true), DIR -1 forward, +1
-// inverse.  In form F the input elements outside [lo, hi) are taken as zero
-// and not read (a zero-padded field needs no zero fill).  Called by all
-// N64_THREADS threads of the block.
-// tw[k] = exp(-2 pi i k / 64).
-constexpr int N64_THREADS = 256;
-template <bool DIGREV_IN, bool COLS, int NLINES, int DIR>
-__device__ __forceinline__ void fft64_lines(float2* s, int line0, const float2* __restrict__ tw, int nlines = NLINES,
-	int lo = 0, int hi = 64) {
-	constexpr int ls = COLS ? 1 : N64_LS, es = COLS ? N64_LS : 1;
-	constexpr float dir = (float)DIR;
-	const unsigned nl = NLINES > 0 ? (unsigned)NLINES : (unsigned)nlines;
+__device__ __forceinline__ void dft8(float2 (&a)[8], float dir) {
+	float2 b[8];
 #pragma unroll
-	for (int step = 0; step < 2; step++) {
-		// F: step 0 gathers 8 i + t and twiddles, step 1 gathers 8 t + i.
-		// G: step 0 gathers 8 t + i and twiddles, step 1 gathers 8 i + t.
-		const bool strided = (step == 0) != DIGREV_IN;
-		const unsigned ntask = nl * 8;
-		// consecutive threads take consecutive lines for column lines, and for
-		// the gather of 8 consecutive elements of row lines (rows are N64_LS
-		// apart: conflict-free), consecutive tasks for the strided gather of row
-		// lines (consecutive elements)
-		const bool lines_fast = COLS || !strided;
-		for (unsigned task = threadIdx.x; task < ntask; task += N64_THREADS) {
-			unsigned L, t;
-			if (lines_fast) {
-				L = task % nl;
-				t = task / nl;
-			} else {
-				L = task >> 3;
-				t = task & 7;
-			}
-			float2* line = s + (line0 + L) * ls;
-			float2 a[8];
+	for (int j = 0; j < 4; j++) {
+		b[j] = make_float2(a[j].x + a[j + 4].x, a[j].y + a[j + 4].y);
+		b[j + 4] = make_float2(a[j].x - a[j + 4].x, a[j].y - a[j + 4].y);
+	}
+	dft8_tail(b, a, dir);
+}
+// the same with a[0], a[1], a[6] and a[7] zero (not read)
+__device__ __forceinline__ void dft8_mid(float2 (&a)[8], float dir) {
+	float2 b[8] = {a[4], a[5], a[2], a[3], make_float2(-a[4].x, -a[4].y), make_float2(-a[5].x, -a[5].y), a[2], a[3]};
+	dft8_tail(b, a, dir);
+}
+// a[i] *= exp(DIR 2 pi i t i / 64); tw[k] = exp(-2 pi i k / 64)
+template <int DIR>
+__device__ __forceinline__ void n64_twiddle(float2 (&a)[8], const float2* tw, int t) {
 #pragma unroll
-			for (int i = 0; i < 8; i++) {
-				const int j = strided ? 8 * i + (int)t : 8 * (int)t + i;
-				if (!DIGREV_IN && step == 0)
-					a[i] = (j >= lo && j < hi) ? line[j * es] : make_float2(0.f, 0.f);
-				else
-					a[i] = line[j * es];
-			}
-			dft8(a, dir);
-			if (step == 0) {
-#pragma unroll
-				for (int i = 1; i < 8; i++) {
-					float2 w = tw[(t * i) & 63u];
-					w.y *= -dir;  // tw holds exp(-...); dir -1 keeps it, +1 conjugates
-					const float2 v = a[i];
-					a[i] = make_float2(v.x * w.x - v.y * w.y, v.x * w.y + v.y * w.x);
-				}
-			}
-#pragma unroll
-			for (int i = 0; i < 8; i++) line[(strided ? 8 * i + (int)t : 8 * (int)t + i) * es] = a[i];
-		}
-		__syncthreads();
+	for (int i = 1; i < 8; i++) {
+		float2 w = tw[t * i];
+		if (DIR > 0) w.y = -w.y;
+		a[i] = make_float2(a[i].x * w.x - a[i].y * w.y, a[i].x * w.y + a[i].y * w.x);
 	}
 }
+// elements at p[es (8 t + i)] (group t) or p[es (8 i + t)] (stride t) of a line
+template <int ES>
+__device__ __forceinline__ void n64_get(float2 (&a)[8], const float2* p) {
+#pragma unroll
+	for (int i = 0; i < 8; i++) a[i] = p[ES * i];
+}
+template <int ES>
+__device__ __forceinline__ void n64_put(float2* p, const float2 (&a)[8]) {
+#pragma unroll
+	for (int i = 0; i < 8; i++) p[ES * i] = a[i];
+}
 
-// (b)-(e) fused for n_f = n_w = 64: one block per work item (item = isa * nw +
-// k as in the other imaging launches).  Dynamic shared memory
-// N64_SMEM_BYTES.  tw64[k] = exp(-2 pi i k / 64), k < 64.
+// (b)-(e) fused for n_f = n_w = 64: one block of N64_THREADS threads per work
+// item (item = isa * nw + k as in the other imaging launches).  Dynamic shared
+// memory N64_SMEM_BYTES.  tw64[k] = exp(-2 pi i k / 64), k < 64.
+//
+// The kernel is bound by the shared-memory wavefronts of its eleven passes
+// over the image, so every element-wise step rides on a pass that holds its
+// operands in registers: the field on the first row transforms' loads (from
+// the OPD itself), |.|^2 and the packing of two PSF rows into one complex row
+// on the last column transforms (a thread takes rows 8t + i and 8t + i + 32 of
+// a column), the unpacking of the half spectrum on the loads of the OTF's
+// columns, the transfer functions between the OTF's last pass and the
+// inverse's first one (both on elements 8i + t of a column: no pass between
+// them), the packing of two image rows on the loads of the inverse's rows (a
+// thread takes the residues t and 8 - t, which hold each other's mirrored
+// frequencies).  Lanes take consecutive lines, so accesses are free of bank
+// conflicts (line stride 65) and a warp shares its twiddles; the pass with the
+// transfer functions takes 8 consecutive frequencies of 4 columns 8 apart
+// instead, so that they are read in 64-byte runs.  Against the 16-pass form
+// with 256 threads (6725 -> 4444 wavefronts an image): 6 WFS of 2820 images
+// 464 -> 355 us, 3 WFS of 808 images 71 -> 54 us.
+constexpr int N64_THREADS = 128;
 constexpr int N64_SMEM_BYTES = (64 * N64_LS + 64) * 8 + 256 * 4;
 // NOPD > 0 fixes the pupil size at compile time (nopd is then ignored).
 template <int NOPD>
 __global__ void __launch_bounds__(N64_THREADS, 6) ints_n64_kernel(PowfsDev P, const WfsDev* __restrict__ wfs, int nw,
 	int nitem, int nopd_rt, float twoinvwvl, const float2* __restrict__ tw64) {
+	static_assert(NOPD == 0 || NOPD == 32, "fixed pupil sizes: 32");
+	constexpr int LS = N64_LS;
 	const int nopd = NOPD > 0 ? NOPD : nopd_rt;
 	extern __shared__ float2 n64_s[];
 	float2* img = n64_s;
-	float2* tw = n64_s + 64 * N64_LS;
+	float2* tw = n64_s + 64 * LS;
 	float* spix = reinterpret_cast<float*>(tw + 64);
-	const int item = blockIdx.x, tid = threadIdx.x;
+	const int item = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	if (item >= nitem) return;
 	const int isa = item / nw;
 	const WfsDev& W = wfs[item % nw];
 	const int pad = (64 - nopd) / 2, no2 = nopd * nopd;
 	if (tid < 64) tw[tid] = tw64[tid];
-	// (b) field, zero-padded (cembed_wvf, maos/wfsints.c:233): only the pupil
-	// square is written; the first transforms read nothing outside it
-	for (int idx = tid; idx < no2; idx += N64_THREADS) {
-		const int y = idx / nopd, x = idx - y * nopd;
-		const float o = __ldg(W.opd + (size_t)isa * no2 + idx), a = __ldg(W.amp + (size_t)isa * no2 + idx);
-		float sn, cs;
-		sincospif(twoinvwvl * o, &sn, &cs);
-		img[(y + pad) * N64_LS + x + pad] = make_float2(a * cs, a * sn);
+	__syncthreads();
+	float2 a[8], b[8];
+	// (b) field, zero-padded (cembed_wvf, maos/wfsints.c:233), and (c) PSF: forward along x on the pupil rows
+	{
+		const float* opd = W.opd + (size_t)isa * no2;
+		const float* amp = W.amp + (size_t)isa * no2;
+		for (int task = tid; task < nopd * 8; task += N64_THREADS) {
+			const int y = task >> 3, t = task & 7;
+			float o[8], m[8];
+#pragma unroll
+			for (int i = 0; i < 8; i++) {
+				const int x = 8 * i + t - pad;
+				const bool in = NOPD ? i >= 2 && i < 6 : x >= 0 && x < nopd;
+				o[i] = in ? __ldg(opd + y * nopd + x) : 0.f;
+				m[i] = in ? __ldg(amp + y * nopd + x) : 0.f;
+			}
+#pragma unroll
+			for (int i = 0; i < 8; i++) {
+				if (NOPD && (i < 2 || i >= 6)) continue;
+				float sn, cs;
+				sincospif(twoinvwvl * o[i], &sn, &cs);
+				a[i] = make_float2(m[i] * cs, m[i] * sn);
+			}
+			if (NOPD) dft8_mid(a, -1.f);
+			else dft8(a, -1.f);
+			n64_twiddle<-1>(a, tw, t);
+			n64_put<8>(img + (y + pad) * LS + t, a);
+		}
 	}
 	__syncthreads();
-	// (c) PSF: forward along x on the pupil rows, along y
-	fft64_lines<false, false, NOPD, -1>(img, pad, tw, nopd, pad, pad + nopd);
-	fft64_lines<false, true, 64, -1>(img, 0, tw, 64, pad, pad + nopd);
+	for (int task = tid; task < nopd * 8; task += N64_THREADS) {
+		const int L = task % nopd, t = task / nopd;
+		float2* p = img + (pad + L) * LS + 8 * t;
+		n64_get<1>(a, p);
+		dft8(a, -1.f);
+		n64_put<1>(p, a);
+	}
+	__syncthreads();
+	// forward along y, the rows outside the pupil being zero
+#pragma unroll 1
+	for (int t = tid >> 6; t < 8; t += 2) {
+		float2* p = img + (tid & 63) + t * LS;
+		if (NOPD) {
+#pragma unroll
+			for (int i = 2; i < 6; i++) a[i] = p[8 * LS * i];
+			dft8_mid(a, -1.f);
+		} else {
+#pragma unroll
+			for (int i = 0; i < 8; i++) {
+				const int y = 8 * i + t;
+				a[i] = y >= pad && y < pad + nopd ? p[8 * LS * i] : make_float2(0.f, 0.f);
+			}
+			dft8(a, -1.f);
+		}
+		n64_twiddle<-1>(a, tw, t);
+		n64_put<8 * LS>(p, a);
+	}
+	__syncthreads();
 	// |.|^2, two real PSF rows per complex row: row r <- (PSF row r) + i (PSF row r + 32)
-	for (int idx = tid; idx < 32 * 64; idx += N64_THREADS) {
-		float2* v = img + (idx >> 6) * N64_LS + (idx & 63);
-		const float2 a = v[0], b = v[32 * N64_LS];
-		v[0] = make_float2(a.x * a.x + a.y * a.y, b.x * b.x + b.y * b.y);
+#pragma unroll 1
+	for (int t = tid >> 6; t < 4; t += 2) {
+		float2* p = img + (tid & 63) + 8 * t * LS;
+		n64_get<LS>(a, p);
+		n64_get<LS>(b, p + 32 * LS);
+		dft8(a, -1.f);
+		dft8(b, -1.f);
+#pragma unroll
+		for (int i = 0; i < 8; i++)
+			p[LS * i] = make_float2(a[i].x * a[i].x + a[i].y * a[i].y, b[i].x * b[i].x + b[i].y * b[i].y);
 	}
 	__syncthreads();
 	// OTF, half spectrum kx = 0..32 (the PSF is real, so OTF(-k) = conj OTF(k)):
 	// forward along kx on the 32 packed rows (digit-reversed inputs)
-	fft64_lines<true, false, 32, -1>(img, 0, tw);
-	// unpack the pairs: row r's spectrum Z = H_r + i H_{r+32}, H_r(kx) = (Z(kx) +
-	// conj Z(-kx)) / 2, H_{r+32}(kx) = (Z(kx) - conj Z(-kx)) / 2i.  H(0) and
-	// H(32) are real, so column 0 carries H(0) + i H(32) and column 32 is free.
-	for (int idx = tid; idx < 32 * 32; idx += N64_THREADS) {
-		const int r = idx >> 5, kx = idx & 31;
-		float2* row = img + r * N64_LS;
-		const float2 z = row[kx], zm = row[kx ? 64 - kx : 32];
-		if (kx) {
-			row[kx] = make_float2(0.5f * (z.x + zm.x), 0.5f * (z.y - zm.y));
-			row[32 * N64_LS + kx] = make_float2(0.5f * (z.y + zm.y), 0.5f * (zm.x - z.x));
-		} else {
-			row[0] = make_float2(z.x, zm.x);
-			row[32 * N64_LS] = make_float2(z.y, zm.y);
-		}
+#pragma unroll 1
+	for (int t = warp; t < 8; t += 4) {
+		float2* p = img + lane * LS + 8 * t;
+		n64_get<1>(a, p);
+		dft8(a, -1.f);
+		n64_twiddle<-1>(a, tw, t);
+		n64_put<1>(p, a);
 	}
 	__syncthreads();
-	// forward along ky on columns 0..31 (digit-reversed inputs): natural OTF
-	fft64_lines<true, true, 32, -1>(img, 0, tw);
-	// x conj(uplink OTF) x ETF / nominal; transfer functions are [fy + 64 fx].
-	// Column 0 holds
-	// Y = O(.,0) + i O(.,32) with O(.,0), O(.,32) the transforms of real
-	// columns; the products for kx = 0 and 32 go to column 32 as X(.,0) + i X(.,32).
+#pragma unroll 1
+	for (int t = warp; t < 8; t += 4) {
+		float2* p = img + lane * LS + t;
+		n64_get<8>(a, p);
+		dft8(a, -1.f);
+		n64_put<8>(p, a);
+	}
+	__syncthreads();
+	// forward along ky on columns kx = 0..31 (digit-reversed inputs), unpacking
+	// the pairs: row r's spectrum Z = H_r + i H_{r+32}, H_r(kx) = (Z(kx) + conj
+	// Z(-kx)) / 2, H_{r+32}(kx) = (Z(kx) - conj Z(-kx)) / 2i.  H(0) and H(32) are
+	// real, so column 0 carries H(0) + i H(32).
+	{
+		const int t = warp, kx = lane;
+		float2* p = img + 8 * t * LS + kx;
+		const float2* pm = img + 8 * t * LS + (kx ? 64 - kx : 32);
+#pragma unroll
+		for (int i = 0; i < 8; i++) {
+			const float2 z = p[LS * i], zm = pm[LS * i];
+			a[i] = kx ? make_float2(0.5f * (z.x + zm.x), 0.5f * (z.y - zm.y)) : make_float2(z.x, zm.x);
+			b[i] = kx ? make_float2(0.5f * (z.y + zm.y), 0.5f * (zm.x - z.x)) : make_float2(z.y, zm.y);
+		}
+		dft8(a, -1.f);
+		n64_twiddle<-1>(a, tw, t);
+		n64_put<LS>(p, a);
+		dft8(b, -1.f);
+		n64_twiddle<-1>(b, tw, t + 4);
+		n64_put<LS>(p + 32 * LS, b);
+	}
+	__syncthreads();
+	// the columns' second half: natural OTF at fy = 8 i + t, x conj(uplink OTF) x
+	// ETF / nominal (transfer functions are [fy + 64 fx]), then the first half
+	// of the inverse along fy on the same elements.  The transfer functions are
+	// transforms of real kernels (uplink PSF, elongated spot, pixel response),
+	// Hermitian to rounding, so each half-spectrum element takes TF itself: the
+	// image is then the real part of the full inverse up to rounding.  Column 0
+	// holds Y = O(.,0) + i O(.,32) with O(.,0), O(.,32) the transforms of real
+	// columns; it goes on as X(.,0) + i X(.,32).
 	{
 		const float2* e1 = P.etfT1 ? P.etfT1 + (size_t)isa * 4096 : nullptr;
 		const float2* e2 = P.etfT2 ? P.etfT2 + (size_t)isa * 4096 : nullptr;
 		const float* nm = P.nominalT ? P.nominalT + (P.nominal_per_sa ? (size_t)isa * 4096 : 0) : nullptr;
-		auto tf = [&](int t) -> float2 {
+		const int t = lane & 7;
+		auto tf1 = [&](int k) {  // transfer function at element k
 			float2 o = make_float2(1.f, 0.f);
-			if (W.lotfT) {
-				const float2 l = __ldg(W.lotfT + t);
-				o = make_float2(l.x, -l.y);
-			}
 			if (e1) {
-				float2 e = __ldg(e1 + t);
+				o = __ldg(e1 + k);
 				if (e2) {
-					const float2 f = __ldg(e2 + t);
-					e = make_float2(e.x * P.etfwt1 + f.x * P.etfwt2, e.y * P.etfwt1 + f.y * P.etfwt2);
+					const float2 f = __ldg(e2 + k);
+					o = make_float2(o.x * P.etfwt1 + f.x * P.etfwt2, o.y * P.etfwt1 + f.y * P.etfwt2);
 				}
-				o = cmul(o, e);
 			} else if (nm) {
-				const float d = __ldg(nm + t);
-				o = make_float2(o.x * d, o.y * d);
+				o.x = __ldg(nm + k);
 			}
-			return o;
+			return W.lotfT ? cmulc(o, __ldg(W.lotfT + k)) : o;
 		};
-		// The transfer functions are transforms of real kernels (uplink PSF,
-		// elongated spot, pixel response), Hermitian to rounding, so each
-		// half-spectrum element takes TF(t) itself: the image is then the real
-		// part of the full inverse up to rounding.
-		for (int t = tid; t < 64 * 32; t += N64_THREADS) {
-			const int fy = t & 63, fx = t >> 6, my = (64 - fy) & 63;
-			if (fx) {
-				float2* v = img + fy * N64_LS + fx;
-				*v = cmul(*v, tf(t));
+		// the same at elements t0 + 8 i, the loads together
+		auto tf = [&](float2 (&o)[8], int t0) {
+			if (e1) {
+#pragma unroll
+				for (int i = 0; i < 8; i++) o[i] = __ldg(e1 + t0 + 8 * i);
+				if (e2) {
+#pragma unroll
+					for (int i = 0; i < 8; i++) {
+						const float2 f = __ldg(e2 + t0 + 8 * i);
+						o[i] = make_float2(o[i].x * P.etfwt1 + f.x * P.etfwt2, o[i].y * P.etfwt1 + f.y * P.etfwt2);
+					}
+				}
 			} else {
-				const float2 y = img[fy * N64_LS], ym = img[my * N64_LS];
-				const float2 o0 = make_float2(0.5f * (y.x + ym.x), 0.5f * (y.y - ym.y));
-				const float2 o32 = make_float2(0.5f * (y.y + ym.y), 0.5f * (ym.x - y.x));
-				const float2 x0 = cmul(o0, tf(fy)), x32 = cmul(o32, tf(fy + 64 * 32));
-				img[fy * N64_LS + 32] = make_float2(x0.x - x32.y, x0.y + x32.x);
+#pragma unroll
+				for (int i = 0; i < 8; i++) o[i] = make_float2(nm ? __ldg(nm + t0 + 8 * i) : 1.f, 0.f);
 			}
+			if (W.lotfT) {
+#pragma unroll
+				for (int i = 0; i < 8; i++) o[i] = cmulc(o[i], __ldg(W.lotfT + t0 + 8 * i));
+			}
+		};
+#pragma unroll 1
+		for (int c = warp; c < 8; c += 4) {
+			const int fx = c + (lane & 24);
+			float2* p = img + t * LS + fx;
+			n64_get<8 * LS>(a, p);
+			tf(b, t + 64 * fx);
+			dft8(a, -1.f);
+			if (c == 0) {  // column 0 is lanes 0..7's: fy's mirror 64 - fy is element 7 - i of lane 8 - t (t = 0: its own 8 - i)
+				float2 ym[8];
+#pragma unroll
+				for (int i = 0; i < 8; i++) {
+					const int src = (lane & 24) | ((8 - t) & 7);
+					const float2 m = make_float2(__shfl_sync(0xffffffffu, a[7 - i].x, src), __shfl_sync(0xffffffffu, a[7 - i].y, src));
+					ym[i] = t ? m : a[(8 - i) & 7];
+				}
+				if (fx == 0) {
+#pragma unroll
+					for (int i = 0; i < 8; i++) {
+						const float2 y = a[i], m = ym[i];
+						const float2 o0 = make_float2(0.5f * (y.x + m.x), 0.5f * (y.y - m.y));
+						const float2 o32 = make_float2(0.5f * (y.y + m.y), 0.5f * (m.x - y.x));
+						const float2 x0 = cmul(o0, b[i]), x32 = cmul(o32, tf1(t + 8 * i + 64 * 32));
+						a[i] = make_float2(x0.x - x32.y, x0.y + x32.x);
+					}
+				} else {
+#pragma unroll
+					for (int i = 0; i < 8; i++) a[i] = cmul(a[i], b[i]);
+				}
+			} else {
+#pragma unroll
+				for (int i = 0; i < 8; i++) a[i] = cmul(a[i], b[i]);
+			}
+			dft8(a, 1.f);
+			n64_twiddle<1>(a, tw, t);
+			n64_put<8 * LS>(p, a);
 		}
 	}
 	__syncthreads();
-	// inverse along fy on columns 1..32: G(y, kx) at digit-reversed rows, column
-	// 32 holding G(., 0) + i G(., 32) (both real)
-	fft64_lines<false, true, 32, 1>(img, 1, tw);
-	// two real image rows per complex row: row r <- a + i b over the full kx
-	// range, a and b the Hermitian extensions of rows r and r + 32
-	for (int idx = tid; idx < 32 * 32; idx += N64_THREADS) {
-		const int r = idx >> 5, kx = idx & 31;
-		float2* row = img + r * N64_LS;
-		if (kx) {
-			const float2 a = row[kx], b = row[32 * N64_LS + kx];
-			row[kx] = make_float2(a.x - b.y, a.y + b.x);
-			row[64 - kx] = make_float2(a.x + b.y, b.x - a.y);
-		} else {
-			const float2 a = row[32], b = row[32 * N64_LS + 32];
-			row[0] = make_float2(a.x, b.x);
-			row[32] = make_float2(a.y, b.y);
-		}
+	// G(y, kx) at digit-reversed rows, column 0 holding G(., 0) + i G(., 32) (both real)
+#pragma unroll 1
+	for (int t = warp; t < 8; t += 4) {
+		float2* p = img + lane + 8 * t * LS;
+		n64_get<LS>(a, p);
+		dft8(a, 1.f);
+		n64_put<LS>(p, a);
 	}
 	__syncthreads();
-	// inverse along fx on the 32 packed rows: image row s (digit-reversed) is the
-	// real part of row s for s < 32, the imaginary part of row s - 32 otherwise
-	fft64_lines<false, false, 32, 1>(img, 0, tw);
+	// inverse along fx on 32 complex rows of two real image rows each: row r is
+	// A + i B over the full kx range, A and B the Hermitian extensions of rows r
+	// and r + 32: at kx < 32 A + i B, at 64 - kx conj A + i conj B
+	{
+		float2* row = img + lane * LS;
+		const int t1 = warp, t2 = warp ? 8 - warp : 4;
+		float2 A1[4], B1[4], A2[4], B2[4];
+#pragma unroll
+		for (int i = 0; i < 4; i++) {
+			A1[i] = row[8 * i + t1];
+			B1[i] = row[32 * LS + 8 * i + t1];
+			A2[i] = row[8 * i + t2];
+			B2[i] = row[32 * LS + 8 * i + t2];
+		}
+		auto lower = [](float2 u, float2 v) { return make_float2(u.x - v.y, u.y + v.x); };
+		auto upper = [](float2 u, float2 v) { return make_float2(u.x + v.y, v.x - u.y); };
+#pragma unroll
+		for (int i = 0; i < 4; i++) {
+			a[i] = lower(A1[i], B1[i]);
+			b[i] = lower(A2[i], B2[i]);
+		}
+		if (warp) {  // 64 - (8 i + t1) = 8 (7 - i) + t2 and the reverse
+#pragma unroll
+			for (int i = 4; i < 8; i++) {
+				a[i] = upper(A2[7 - i], B2[7 - i]);
+				b[i] = upper(A1[7 - i], B1[7 - i]);
+			}
+		} else {  // 64 - 8 i = 8 (8 - i), kx = 0 and 32 packed; 64 - (8 i + 4) = 8 (7 - i) + 4
+			a[0] = make_float2(A1[0].x, B1[0].x);
+			a[4] = make_float2(A1[0].y, B1[0].y);
+#pragma unroll
+			for (int i = 5; i < 8; i++) a[i] = upper(A1[8 - i], B1[8 - i]);
+#pragma unroll
+			for (int i = 4; i < 8; i++) b[i] = upper(A2[7 - i], B2[7 - i]);
+		}
+		dft8(a, 1.f);
+		n64_twiddle<1>(a, tw, t1);
+		n64_put<8>(row + t1, a);
+		dft8(b, 1.f);
+		n64_twiddle<1>(b, tw, t2);
+		n64_put<8>(row + t2, b);
+	}
+	__syncthreads();
+	// image row s (digit-reversed) is the real part of row s for s < 32, the
+	// imaginary part of row s - 32 otherwise
+#pragma unroll 1
+	for (int t = warp; t < 8; t += 4) {
+		float2* p = img + lane * LS + 8 * t;
+		n64_get<1>(a, p);
+		dft8(a, 1.f);
+		n64_put<1>(p, a);
+	}
+	__syncthreads();
 	// (d) pixels (bilinear map) and noise, one thread per pixel
 	const int npix = P.npix;
 	const int* sidx = P.simap_idx + (P.simap_per_sa ? (size_t)isa * npix * 4 : 0);

@@ -1,0 +1,77 @@
+"""Imaging at FFT 64 against plain FP64 transforms.
+
+FFT 64 (ints_n64_kernel): pupils of 16, 32 and 64 points (the fixed size and
+the general one), a DTF nominal or an ETF with an uplink OTF, and pixel counts
+below, at and above a block's threads.  Tolerance: noise-free intensities
+within 1e-5 of the subaperture total, the bar of the other imaging tests."""
+import math
+
+import numpy as np
+import pytest
+
+from tests.conftest import cuda_available
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not cuda_available(), reason="needs a CUDA GPU")]
+
+
+def _kernel_tf(rng, shape, N):
+    """Transfer function of a random real kernel around the origin."""
+    k = np.zeros(shape + (N, N))
+    for dy in (-1, 0, 1):
+        for dx in (-1, 0, 1):
+            k[..., dy % N, dx % N] = rng.uniform(0.2, 1.0, shape)
+    return np.fft.fft2(k / 9)
+
+
+@pytest.mark.parametrize("nopd,pix", [(32, 5), (32, 12), (32, 16), (16, 8), (64, 11)])
+@pytest.mark.parametrize("lgs", [False, True])
+def test_fft64_images_match_plain(nopd, pix, lgs):
+    import torch
+    from maos_b200 import shwfs
+    rng = np.random.default_rng(nopd * 100 + pix)
+    N, nsa, nllt, wvl = 64, 5, nopd, 0.6e-6  # an LLT pupil has the subapertures' sampling
+    npix = pix * pix
+    ctx = shwfs.Context(0)
+    ip = ctx.powfs_add(nsa=nsa, nopd=nopd, embfac=N // nopd, notf=N, pixpsax=pix, pixpsay=pix, pixthetax=1e-6,
+                       pixthetay=1e-6, wvl=wvl, dsa=0.5, dx=0.5 / nopd, areascale=1.0, hs=90e3 if lgs else math.inf,
+                       has_etf=int(lgs), has_llt=int(lgs), llt_nx=nllt if lgs else 0, gradtype=shwfs.SHWFS_GRAD_COG,
+                       sigmatch=1)
+    amp = rng.uniform(0, 1, (nsa, nopd, nopd))
+    amp /= np.sqrt((amp ** 2).sum((1, 2), keepdims=True))
+    ctx.powfs_set_geom(ip, np.zeros(nsa), np.zeros(nsa), amp, np.ones(nsa))
+    idx = rng.integers(0, N * N, (npix, 4))
+    idx[rng.uniform(size=idx.shape) < 0.2] = -1
+    wt = rng.uniform(0, 1, (npix, 4))
+    ctx.powfs_set_simap(ip, idx, wt)
+    if lgs:
+        tf = _kernel_tf(rng, (nsa,), N)
+        lltamp = rng.uniform(0, 1, (nllt, nllt))
+        lltamp /= np.sqrt((lltamp ** 2).sum())
+        ctx.powfs_set_etf(ip, tf.reshape(nsa, -1))
+        ctx.powfs_set_lltamp(ip, lltamp)
+    else:
+        tf = np.zeros((1, N, N))
+        tf[0] = np.cos(np.arange(N) * 2 * np.pi / N)[:, None] * 0.3 + np.cos(np.arange(N) * 4 * np.pi / N)[None] * 0.2 + 1
+        ctx.powfs_set_nominal(ip, tf)
+    iw = ctx.wfs_add(ipowfs=ip, thetax=0.0, thetay=0.0, hs=90e3 if lgs else math.inf, hc=0.0, misregx=0.0, misregy=0.0,
+                     sigsim=700.0, wvlwt=1.0, noisy=0)
+    opd = rng.normal(0, 1.5e-7, (nsa, nopd, nopd)).astype(np.float32)
+    llt = rng.normal(0, 1.5e-7, (nllt, nllt)).astype(np.float32)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    ints, grad = torch.full((nsa * npix,), -1.0, device="cuda"), torch.zeros(2 * nsa, device="cuda")
+    d_opd, d_llt = dev(opd), dev(llt)
+    torch.cuda.synchronize()
+    ctx.ints_grad_dev(iw, 0, d_opd, d_llt if lgs else None, ints, grad)
+    ctx.sync()
+    psf = lambda a, o: np.abs(np.fft.fft2(a * np.exp(2j * np.pi / wvl * o), s=(N, N))) ** 2  # noqa: E731
+    otf = np.fft.fft2(psf(amp, opd.astype(float)))
+    if lgs:
+        otf = otf * np.conj(np.fft.fft2(psf(lltamp, llt.astype(float)) / N ** 2))
+    img = np.fft.ifft2(otf * tf).real * N * N
+    scale = 700.0 / (nopd * N) ** 2 / N ** 2
+    flat = img.reshape(nsa, -1)
+    ref = np.stack([(np.where(idx >= 0, flat[k][np.maximum(idx, 0)], 0) * wt).sum(1) * scale for k in range(nsa)])
+    total = np.abs(flat).sum(1, keepdims=True) * scale
+    got = ints.double().cpu().numpy().reshape(nsa, npix)
+    assert (np.abs(got - ref) / total).max() <= 1e-5
+    ctx.close()
