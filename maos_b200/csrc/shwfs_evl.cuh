@@ -25,33 +25,40 @@ struct EvlRaster {
 // (1) loc_calc_ptt_stride (math/loc.c:653-704) sums over the aperture, per
 // direction: s = {sum a o^2, sum a o, sum a o x, sum a o y}, FP64; grid
 // (ceil(nslot / EVL_SUM_TILES), nevl), 256 threads (one point of a tile
-// each), EVL_SUM_TILES tiles per block with all their loads in flight; sums
-// zeroed before the launch.
-constexpr int EVL_SUM_TILES = 8;
-__global__ void __launch_bounds__(256) evl_sums_kernel(EvlRaster R, const float* __restrict__ opd, double* sums) {
+// each), EVL_SUM_BATCH tiles' loads in flight; sums zeroed before the launch.
+// A point's position is its tile's origin plus an offset that is the thread's
+// own, which enters once, at the end: two FP64 fused multiply-adds a point
+// instead of the index arithmetic of its raster position (three directions of
+// 30 m at 1/64 m: 30 -> 24 us, bound by the loads' latency).
+constexpr int EVL_SUM_TILES = 32, EVL_SUM_BATCH = 8;
+__global__ void __launch_bounds__(256) evl_sums_kernel(EvlRaster R, const double* __restrict__ torigx,
+	const double* __restrict__ torigy, const float* __restrict__ opd, double* sums) {
 	const int e = blockIdx.y, p = threadIdx.x;
 	const float* o = opd + (size_t)e * R.nslot * 256;
-	const int slot0 = blockIdx.x * EVL_SUM_TILES;
-	float av[EVL_SUM_TILES], ov[EVL_SUM_TILES];
-#pragma unroll
-	for (int k = 0; k < EVL_SUM_TILES; k++) {
-		const int slot = slot0 + k;
-		const size_t i = (size_t)slot * 256 + p;
-		av[k] = slot < R.nslot ? __ldg(R.amp + i) : 0.f;
-		ov[k] = slot < R.nslot ? __ldg(o + i) : 0.f;
-	}
 	double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
+#pragma unroll 1
+	for (int b = 0; b < EVL_SUM_TILES; b += EVL_SUM_BATCH) {
+		const int slot0 = blockIdx.x * EVL_SUM_TILES + b;
+		float av[EVL_SUM_BATCH], ov[EVL_SUM_BATCH];
 #pragma unroll
-	for (int k = 0; k < EVL_SUM_TILES; k++) {
-		if (av[k] == 0.f) continue;
-		const int tile = R.slot_tile[slot0 + k];
-		const int X = (tile % R.ntx) * 16 + (p & 15), Y = (tile / R.ntx) * 16 + (p >> 4);
-		const double v = ov[k], a = (double)av[k] * v;
-		s0 += a * v;
-		s1 += a;
-		s2 += a * (R.ox + X * R.dx);
-		s3 += a * (R.oy + Y * R.dx);
+		for (int k = 0; k < EVL_SUM_BATCH; k++) {
+			const int slot = slot0 + k;
+			const size_t i = (size_t)slot * 256 + p;
+			av[k] = slot < R.nslot ? __ldg(R.amp + i) : 0.f;
+			ov[k] = slot < R.nslot ? __ldg(o + i) : 0.f;
+		}
+#pragma unroll
+		for (int k = 0; k < EVL_SUM_BATCH; k++) {
+			const int slot = min(slot0 + k, R.nslot - 1);
+			const double v = av[k] != 0.f ? ov[k] : 0.f, a = (double)av[k] * v;
+			s0 += a * v;
+			s1 += a;
+			s2 += a * __ldg(torigx + slot);
+			s3 += a * __ldg(torigy + slot);
+		}
 	}
+	s2 += s1 * ((p & 15) * R.dx);
+	s3 += s1 * ((p >> 4) * R.dx);
 	__shared__ double red[4][8];
 #pragma unroll
 	for (int off = 16; off > 0; off >>= 1) {
@@ -323,6 +330,176 @@ __global__ void __launch_bounds__(EVL_THREADS, 4) evl_psf_cols_kernel(const floa
 		if (ay >= 0) P[ay] += v.x * v.x + v.y * v.y;
 	};
 	evl_fft_smem<N, 1>(s_col, tw, offy, offy + nY, acc);
+}
+
+// (3f), (4f) The same two dimensions for crops of at most EVL_FOLD_M pixels
+// from lines of 512 or more.  Such a crop is EVL_FOLD_M consecutive
+// frequencies k = k1 + 16 k2, |k| <= 128, of the N-point transform, so the
+// transform needs two radix-16 passes and one sum instead of all its stages:
+// with T = N / 16, Q = N / 256 and n = T i + t, t = Q j + r,
+//   X[k] = sum_r w_T^(r k2) sum_j w_16^(j k2) { w_N^(t k1) sum_i w_16^(i k1) x[T i + t] }.
+// A thread (t) takes its 16 points T i + t straight from global memory
+// (consecutive threads, consecutive points), one exchange through shared
+// memory regroups them by j, and the sum over r is a reduce-scatter of the
+// 16 values of Q lanes by shuffles, which leaves each thread the outputs
+// k2 = r (16 / Q) + i.  Full transforms of 4096 points take four passes
+// through shared memory instead, of which 15/16 of the last one's outputs are
+// dropped at 256 pixels.  Blocks are persistent (their twiddle tables are
+// made once) and take EvlFold<N>::LPB lines at a time.  Measured on three
+// directions of the 30 m aperture at 1/64 m (5763 rows of 4096): rows 141 ->
+// 96 us, columns 23 -> 20 us a wavelength.  What bounds the rows now: the
+// latency of the gathers at 24 warps per SM (issue 59 %).
+constexpr int EVL_FOLD_M = 256, EVL_FOLD_THREADS = 256, EVL_FOLD_BLOCKS = 3;  // 3 blocks of 66 KB per SM
+template <int N>
+struct EvlFold {
+	static constexpr int T = N / 16, Q = N / 256, LPB = EVL_FOLD_THREADS / T;
+	static constexpr int SMEM = (16 * T + 16 * EVL_FOLD_THREADS + 16 * Q) * (int)sizeof(float2);
+};
+
+template <int N, class In, class Out>
+__device__ __forceinline__ void evl_fold_lines(float2* smem, const float2* __restrict__ tw, int nline, In in, Out out) {
+	using F = EvlFold<N>;
+	constexpr int T = F::T, Q = F::Q;
+	float2* w1 = smem;             // [k1][t] w_N^(t k1)
+	float2* w2 = smem + 16 * T;    // [k2][r] w_T^(r k2), k2 = 0..7, -8..-1
+	float2* ex = w2 + 16 * Q;      // per line [k1][t]
+	const int tid = threadIdx.x, t = tid % T, ln = tid / T, j = t / Q, r = t % Q;
+	for (int k = tid; k < 16 * T; k += EVL_FOLD_THREADS) w1[k] = __ldg(tw + ((k / T) * (k % T) & (N - 1)));
+	for (int k = tid; k < 16 * Q; k += EVL_FOLD_THREADS) {
+		const int k2 = k / Q < 8 ? k / Q : k / Q - 16;
+		w2[k] = __ldg(tw + (16 * (k % Q) * k2 & (N - 1)));
+	}
+	__syncthreads();
+	float2* x = ex + ln * N;
+	for (int l0 = blockIdx.x * F::LPB; l0 < nline; l0 += gridDim.x * F::LPB) {
+		const int line = l0 + ln;
+		float2 v[16];
+		in(line, t, v);
+		fft_reg<-1, 16>(v);
+#pragma unroll
+		for (int k = 0; k < 16; k++) x[k * T + t] = k ? cmul(v[k], w1[k * T + t]) : v[k];
+		__syncthreads();
+#pragma unroll
+		for (int i = 0; i < 16; i++) v[i] = x[j * T + Q * i + r];  // k1 = j
+		__syncthreads();
+		fft_reg<-1, 16>(v);
+#pragma unroll
+		for (int k = 1; k < 16; k++) v[k] = cmul(v[k], w2[k * Q + r]);
+		// sum over the Q lanes r; each keeps 16 / Q of the k2
+		int n = 16;
+#pragma unroll
+		for (int s = Q / 2; s >= 1; s >>= 1) {
+			n >>= 1;
+			const bool up = (r & s) != 0;
+#pragma unroll
+			for (int i = 0; i < 8; i++) {
+				if (i < n) {
+					const float2 give = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+					v[i] = make_float2(keep.x + __shfl_xor_sync(0xffffffffu, give.x, s),
+						keep.y + __shfl_xor_sync(0xffffffffu, give.y, s));
+				}
+			}
+		}
+#pragma unroll
+		for (int i = 0; i < 16 / Q; i++) {
+			const int k2 = r * (16 / Q) + i;
+			out(line, j + 16 * (k2 < 8 ? k2 : k2 - 16), v[i]);
+		}
+	}
+}
+
+// rows: line = direction * nY + Y, the field of raster row Y; T as evl_psf_rows_kernel writes it
+template <int N>
+__global__ void __launch_bounds__(EVL_FOLD_THREADS, EVL_FOLD_BLOCKS) evl_fold_rows_kernel(EvlRaster Ra,
+	const float* __restrict__ opd, const double* __restrict__ coeff, int pttr, float twoinvwvl, int offx, int h,
+	const float2* __restrict__ tw, float2* __restrict__ T, int nYp, int nevl) {
+	extern __shared__ float2 s_fold[];
+	constexpr int S = N / 16;
+	const int nY = Ra.nY, nline = nevl * nY;
+	auto in = [&](int line, int t, float2 (&v)[16]) {
+		const bool on = line < nline;
+		const int e = on ? line / nY : 0, Y = on ? line - e * nY : 0;
+		const int* trow = Ra.tile_slot + (Y >> 4) * Ra.ntx;
+		const float* o = opd + (size_t)e * Ra.nslot * 256;
+		const int py = (Y & 15) * 16;
+		double cy = 0, cx = 0;  // piston, tip and tilt on this row: cy + cx X
+		if (pttr) {
+			cx = coeff[e * 3 + 1];
+			cy = coeff[e * 3] + cx * Ra.ox + coeff[e * 3 + 2] * (Ra.oy + Y * Ra.dx);
+			cx *= Ra.dx;
+		}
+#pragma unroll
+		for (int i0 = 0; i0 < 16; i0 += 8) {
+			int pp[8];
+			float av[8], ov[8];
+#pragma unroll
+			for (int i = 0; i < 8; i++) {
+				const int X = S * (i0 + i) + t - offx;
+				pp[i] = -1;
+				if (on && X >= 0 && X < Ra.nX) {
+					const int slot = __ldg(trow + (X >> 4));
+					if (slot >= 0) pp[i] = slot * 256 + py + (X & 15);
+				}
+			}
+#pragma unroll
+			for (int i = 0; i < 8; i++) {
+				av[i] = pp[i] >= 0 ? __ldg(Ra.amp + pp[i]) : 0.f;
+				ov[i] = pp[i] >= 0 ? __ldg(o + pp[i]) : 0.f;
+			}
+#pragma unroll
+			for (int i = 0; i < 8; i++) {
+				v[i0 + i] = make_float2(0.f, 0.f);
+				if (av[i] != 0.f) {
+					float p = ov[i];
+					if (pttr) p = (float)((double)p - (cy + cx * (S * (i0 + i) + t - offx)));
+					float sn, cs;
+					sincospif(twoinvwvl * p, &sn, &cs);  // exp(i 2 pi p / wvl)
+					v[i0 + i] = make_float2(av[i] * cs, av[i] * sn);
+				}
+			}
+		}
+	};
+	auto out = [&](int line, int k, float2 v) {
+		const int ax = k + h;
+		if (line >= nline || ax < 0 || ax >= 2 * h) return;
+		const int e = line / nY, Y = line - e * nY;
+		T[((size_t)e * (2 * h) + ax) * nYp + Y] = v;
+	};
+	evl_fold_lines<N>(s_fold, tw, nline, in, out);
+}
+
+// columns: line = direction * 2h + crop column, added to the sums as evl_psf_cols_kernel does
+template <int N>
+__global__ void __launch_bounds__(EVL_FOLD_THREADS, EVL_FOLD_BLOCKS) evl_fold_cols_kernel(const float2* __restrict__ T,
+	int nY, int nYp, int offy, int h, const float2* __restrict__ tw, float* __restrict__ psf, int nevl) {
+	extern __shared__ float2 s_fold[];
+	constexpr int S = N / 16;
+	const int nline = nevl * 2 * h;
+	auto in = [&](int line, int t, float2 (&v)[16]) {
+		const float2* x = T + (size_t)line * nYp;
+#pragma unroll
+		for (int i = 0; i < 16; i++) {
+			const int Y = S * i + t - offy;
+			v[i] = line < nline && Y >= 0 && Y < nY ? __ldg(x + Y) : make_float2(0.f, 0.f);
+		}
+	};
+	auto out = [&](int line, int k, float2 v) {
+		const int ay = k + h;
+		if (line < nline && ay >= 0 && ay < 2 * h) psf[(size_t)line * (2 * h) + ay] += v.x * v.x + v.y * v.y;
+	};
+	evl_fold_lines<N>(s_fold, tw, nline, in, out);
+}
+
+// The PSF sum of one direction (crop column major) as the caller's image, x
+// fastest: out[ax + n ay] = psf[ax n + ay]; blocks of 32 x 8 threads, 32 x 32 tiles.
+__global__ void __launch_bounds__(256) evl_image_kernel(const float* __restrict__ psf, int n, float* __restrict__ out) {
+	__shared__ float s[32][33];
+	const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32, tx = threadIdx.x, ty = threadIdx.y;
+	for (int k = ty; k < 32; k += 8)
+		if (x0 + k < n && y0 + tx < n) s[k][tx] = psf[(size_t)(x0 + k) * n + y0 + tx];
+	__syncthreads();
+	for (int k = ty; k < 32; k += 8)
+		if (y0 + k < n && x0 + tx < n) out[(size_t)(y0 + k) * n + x0 + tx] = s[tx][k];
 }
 
 // (5) OPD of one direction in aperture order.

@@ -32,6 +32,9 @@ struct EvlState {
 	int pttr = 0;
 	long nframe = 0;
 	DevBuf<float2> T;
+	DevBuf<float> img;              // one PSF as an image (shwfs_evl_psf_get), and its pinned copy
+	float* img_h = nullptr;
+	size_t img_h_n = 0;
 	int queued = 0;
 };
 
@@ -53,6 +56,8 @@ static void evl_free(shwfs_ctx* ctx) {
 		p.tw.free_();
 		p.psf.free_();
 	}
+	E->img.free_();
+	if (E->img_h) cudaFreeHost(E->img_h);
 	if (E->sums_h) cudaFreeHost(E->sums_h);
 	delete E;
 	ctx->evl = nullptr;
@@ -238,8 +243,29 @@ int shwfs_evl_psf_reset(shwfs_ctx* ctx) {
 
 }  // extern "C"
 
+// The two-pass transforms serve crops of at most 256 pixels; larger ones keep
+// more outputs than their radix-16 passes form and take the full transforms.
+template <int N>
+static int evl_launch_fold(shwfs_ctx* ctx, EvlState& E, EvlPsf& P, int nevl) {
+	using F = EvlFold<N>;
+	CK(cudaFuncSetAttribute(evl_fold_rows_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, F::SMEM));
+	CK(cudaFuncSetAttribute(evl_fold_cols_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, F::SMEM));
+	const long most = (long)sm_count(ctx) * EVL_FOLD_BLOCKS;
+	auto grid = [&](long lines) { return (unsigned)std::min(most, (lines + F::LPB - 1) / F::LPB); };
+	evl_fold_rows_kernel<N><<<grid((long)nevl * E.nY), EVL_FOLD_THREADS, F::SMEM, ctx->stream>>>(evl_raster(E), E.opd.p,
+		E.coeff.p, E.pttr, (float)(2.0 / P.wvl), P.offx, P.h, P.tw.p, E.T.p, E.nY, nevl);
+	CK(cudaGetLastError());
+	evl_fold_cols_kernel<N><<<grid((long)nevl * 2 * P.h), EVL_FOLD_THREADS, F::SMEM, ctx->stream>>>(E.T.p, E.nY, E.nY,
+		P.offy, P.h, P.tw.p, P.psf.p, nevl);
+	CK(cudaGetLastError());
+	return 0;
+}
+
 template <int N>
 static int evl_launch_psf(shwfs_ctx* ctx, EvlState& E, EvlPsf& P, int nevl) {
+	if constexpr (N >= 512) {
+		if (P.psfsize <= EVL_FOLD_M) return evl_launch_fold<N>(ctx, E, P, nevl);
+	}
 	constexpr int R = 4096 / N;  // rows per block: 512 radix-8 groups, one per thread
 	const size_t smem_r = (size_t)R * evl_row_len<N>() * sizeof(float2), smem_c = (size_t)evl_row_len<N>() * sizeof(float2);
 	if (smem_r > 48 * 1024)
@@ -293,7 +319,8 @@ int shwfs_evl_queue(shwfs_ctx* ctx, int isim, int do_psf) {
 	{
 		StageMark m(ctx, SHWFS_STAGE_POST);
 		const unsigned nblk = (unsigned)((E.nslot + EVL_SUM_TILES - 1) / EVL_SUM_TILES);
-		evl_sums_kernel<<<dim3(nblk, nevl), 256, 0, ctx->stream>>>(evl_raster(E), E.opd.p, E.sums.p);
+		evl_sums_kernel<<<dim3(nblk, nevl), 256, 0, ctx->stream>>>(evl_raster(E), E.torigx.p, E.torigy.p, E.opd.p,
+			E.sums.p);
 		CK(cudaGetLastError());
 	}
 	// (c) PSF sums (psfcomp_r, cuda/sim/perfevl.cu:255-300)
@@ -366,16 +393,28 @@ int shwfs_evl_psf_get(shwfs_ctx* ctx, int ievl, int iwvl, double* psf, long* nfr
 		return ctx ? fail(ctx, SHWFS_EINVAL, "evl_psf_get: bad arguments") : SHWFS_EINVAL;
 	int r = set_device(ctx);
 	if (r) return r;
-	const EvlPsf& P = ctx->evl->psf[iwvl];
+	EvlState& E = *ctx->evl;
+	const EvlPsf& P = E.psf[iwvl];
 	const int n = P.psfsize;
-	std::vector<float> h((size_t)n * n, 0.f);
-	if (P.psf.p) {
-		CK(cudaMemcpyAsync(h.data(), P.psf.p + (size_t)ievl * n * n, sizeof(float) * n * n, cudaMemcpyDeviceToHost,
-			ctx->stream));
+	const size_t nn = (size_t)n * n;
+	if (!P.psf.p) {
+		memset(psf, 0, sizeof(double) * nn);
+	} else {
+		if (E.img.n < nn && (r = dev_alloc(ctx, E.img, nn))) return r;
+		if (E.img_h_n < nn) {
+			if (E.img_h) cudaFreeHost(E.img_h);
+			E.img_h = nullptr;
+			E.img_h_n = 0;
+			CK(cudaMallocHost(&E.img_h, sizeof(float) * nn));
+			E.img_h_n = nn;
+		}
+		const int nb = (n + 31) / 32;
+		evl_image_kernel<<<dim3(nb, nb), dim3(32, 8), 0, ctx->stream>>>(P.psf.p + (size_t)ievl * nn, n, E.img.p);
+		CK(cudaGetLastError());
+		CK(cudaMemcpyAsync(E.img_h, E.img.p, sizeof(float) * nn, cudaMemcpyDeviceToHost, ctx->stream));
 		CK(cudaStreamSynchronize(ctx->stream));
+		f32_to_f64(E.img_h, psf, nn);
 	}
-	for (int ax = 0; ax < n; ax++)
-		for (int ay = 0; ay < n; ay++) psf[ax + (size_t)ay * n] = h[(size_t)ax * n + ay];
 	if (nframe) *nframe = ctx->evl->nframe;
 	return 0;
 }

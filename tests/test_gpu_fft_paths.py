@@ -1,9 +1,14 @@
-"""Imaging at FFT 64 against plain FP64 transforms.
+"""Imaging at FFT 64 and the cropped science PSF against plain FP64 transforms.
 
 FFT 64 (ints_n64_kernel): pupils of 16, 32 and 64 points (the fixed size and
 the general one), a DTF nominal or an ETF with an uplink OTF, and pixel counts
 below, at and above a block's threads.  Tolerance: noise-free intensities
-within 1e-5 of the subaperture total, the bar of the other imaging tests."""
+within 1e-5 of the subaperture total, the bar of the other imaging tests.
+
+Science PSF: crops of at most 256 pixels run the two-pass transforms
+(evl_fold_rows_kernel, evl_fold_cols_kernel) for lines of 512 to 4096 points,
+larger crops the full ones; apertures of odd and even width.  Tolerance:
+within 2e-5 of the peak, as the science path's reference test."""
 import math
 
 import numpy as np
@@ -74,4 +79,50 @@ def test_fft64_images_match_plain(nopd, pix, lgs):
     total = np.abs(flat).sum(1, keepdims=True) * scale
     got = ints.double().cpu().numpy().reshape(nsa, npix)
     assert (np.abs(got - ref) / total).max() <= 1e-5
+    ctx.close()
+
+
+@pytest.mark.parametrize("N,ps,nx", [(512, 256, 301), (512, 258, 301), (1024, 50, 1024), (2048, 256, 130), (4096, 16, 701),
+                                     (4096, 256, 700)])
+@pytest.mark.parametrize("pttr", [0, 1])
+def test_cropped_psf_matches_plain(N, ps, nx, pttr):
+    from maos_b200 import shwfs
+    rng = np.random.default_rng(N + ps)
+    dx, wvl, nxs, sdx = 1 / 32, 1.5e-6, 256, 0.25
+    ix, iy = np.meshgrid(np.arange(nx), np.arange(nx - 7))
+    keep = (ix - nx / 2) ** 2 + (iy - nx / 2) ** 2 <= (nx / 2) ** 2
+    keep[0, 0] = keep[-1, -1] = keep[0, -1] = True  # the whole bounding box
+    ix, iy = ix[keep], iy[keep]
+    x, y = (ix - nx / 2) * dx, (iy - nx / 2) * dx
+    amp = rng.uniform(0.5, 1, len(x))
+    amp /= amp.sum()
+    ctx = shwfs.Context(0)
+    ctx.set_dt(1 / 800)
+    t = np.arange(nxs) * 2 * np.pi / nxs
+    scr = 2e-7 * (np.cos(3 * t)[None] + np.sin(2 * t)[:, None] + np.cos(7 * t[None] + 5 * t[:, None]))
+    ctx.atm_set([dict(nx=nxs, ny=nxs, dx=sdx, ox=-nxs / 2 * sdx, oy=-nxs / 2 * sdx, ht=0.0, vx=0.0, vy=0.0, alpha=1.0)], [scr])
+    ctx.evl_set_aper(x, y, dx, amp)
+    ctx.evl_add_dir(0.0, 0.0)
+    ctx.evl_set_psf([wvl], [N], [ps], pttr=pttr)
+    ctx.evl_queue(0, do_psf=True)
+    wfe, coeff = ctx.evl_sync()
+    got, n = ctx.evl_psf(0, 0)
+    assert n == 1
+    u, v = x / sdx + nxs / 2, y / sdx + nxs / 2
+    ju, jv = np.floor(u).astype(int), np.floor(v).astype(int)
+    wu, wv = u - ju, v - jv
+    at = lambda a, b: scr[a % nxs, b % nxs]  # noqa: E731
+    o = (at(jv, ju) * (1 - wu) + at(jv, ju + 1) * wu) * (1 - wv) + (at(jv + 1, ju) * (1 - wu) + at(jv + 1, ju + 1) * wu) * wv
+    B = np.stack([np.ones_like(x), x, y])
+    c = np.linalg.solve((B * amp) @ B.T, (B * amp) @ o)
+    assert np.allclose(coeff[0], c, rtol=0, atol=1e-4 * np.abs(c).max())
+    if pttr:
+        o = o - c @ B
+    E = np.zeros((nx, nx - 7), complex)
+    E[ix, iy] = amp * np.exp(2j * np.pi / wvl * o)
+    h = ps // 2
+    f = np.concatenate([np.arange(N - h, N), np.arange(h)])
+    F = np.fft.fft(np.fft.fft(E, n=N, axis=0)[f], n=N, axis=1)[:, f]
+    ref = np.abs(F) ** 2
+    assert np.abs(got - ref).max() <= 2e-5 * ref.max()
     ctx.close()
