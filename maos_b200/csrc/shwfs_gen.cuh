@@ -408,22 +408,20 @@ __device__ __forceinline__ void dft8_tail(float2 (&b)[8], float2 (&a)[8], float 
 #pragma unroll
 	for (int g = 0; g < 2; g++) {
 		const float2 c0 = b[4 * g], c1 = b[4 * g + 1], c2 = b[4 * g + 2], c3 = b[4 * g + 3];
-		const float2 s0 = make_float2(c0.x + c2.x, c0.y + c2.y), d0 = make_float2(c0.x - c2.x, c0.y - c2.y);
-		const float2 s1 = make_float2(c1.x + c3.x, c1.y + c3.y), d1 = make_float2(c1.x - c3.x, c1.y - c3.y);
+		const float2 s0 = cadd(c0, c2), d0 = csub(c0, c2), s1 = cadd(c1, c3), d1 = csub(c1, c3);
 		const float2 d1r = make_float2(-dir * d1.y, dir * d1.x);  // d1 * (dir i)
-		a[g] = make_float2(s0.x + s1.x, s0.y + s1.y);                // X[0] / X[1]
-		a[g + 2] = make_float2(d0.x + d1r.x, d0.y + d1r.y);          // X[2] / X[3]
-		a[g + 4] = make_float2(s0.x - s1.x, s0.y - s1.y);            // X[4] / X[5]
-		a[g + 6] = make_float2(d0.x - d1r.x, d0.y - d1r.y);          // X[6] / X[7]
+		a[g] = cadd(s0, s1);                                  // X[0] / X[1]
+		a[g + 2] = make_float2(d0.x + d1r.x, d0.y + d1r.y);  // X[2] / X[3]
+		a[g + 4] = csub(s0, s1);                              // X[4] / X[5]
+		a[g + 6] = make_float2(d0.x - d1r.x, d0.y - d1r.y);  // X[6] / X[7]
 	}
 }
-
 __device__ __forceinline__ void dft8(float2 (&a)[8], float dir) {
 	float2 b[8];
 #pragma unroll
 	for (int j = 0; j < 4; j++) {
-		b[j] = make_float2(a[j].x + a[j + 4].x, a[j].y + a[j + 4].y);
-		b[j + 4] = make_float2(a[j].x - a[j + 4].x, a[j].y - a[j + 4].y);
+		b[j] = cadd(a[j], a[j + 4]);
+		b[j + 4] = csub(a[j], a[j + 4]);
 	}
 	dft8_tail(b, a, dir);
 }
@@ -473,7 +471,7 @@ __device__ __forceinline__ void n64_put(float2* p, const float2 (&a)[8]) {
 // transfer functions takes 8 consecutive frequencies of 4 columns 8 apart
 // instead, so that they are read in 64-byte runs.  Against the 16-pass form
 // with 256 threads (6725 -> 4444 wavefronts an image): 6 WFS of 2820 images
-// 464 -> 355 us, 3 WFS of 808 images 71 -> 54 us.
+// 464 -> 342 us, 3 WFS of 808 images 71 -> 54 us.
 constexpr int N64_THREADS = 128;
 constexpr int N64_SMEM_BYTES = (64 * N64_LS + 64) * 8 + 256 * 4;
 // NOPD > 0 fixes the pupil size at compile time (nopd is then ignored).

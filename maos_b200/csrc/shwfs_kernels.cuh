@@ -795,8 +795,9 @@ __device__ __forceinline__ void grad_from_pixels(const float (&pix)[NPQ], int np
 			const int p = lane + 32 * q;
 			if (p < npix) {
 				const double v = pix[q];
-				sx += (double)__ldg(mtche + 2 * p) * v;
-				sy += (double)__ldg(mtche + 2 * p + 1) * v;
+				const float2 m = __ldg(reinterpret_cast<const float2*>(mtche) + p);  // 8-byte aligned: 2 npix floats a subaperture
+				sx += (double)m.x * v;
+				sy += (double)m.y * v;
 				si += v;
 			}
 		}
@@ -918,19 +919,22 @@ __device__ __forceinline__ void ints_n32_pixels(const PowfsDev& P, const WfsDev&
 	const float* psf) {
 	// pixel sampling (mkh bilinear map, up to 4 taps per pixel)
 	const int npix = P.npix;
-	const int* sidx = P.simap_idx + (P.simap_per_sa ? (size_t)isa * npix * 4 : 0);
-	const float* swt = P.simap_wt + (P.simap_per_sa ? (size_t)isa * npix * 4 : 0);
+	// a pixel's 4 map entries are one 16-byte row (cudaMalloc'd, 4 entries per
+	// pixel); a missing tap (index < 0) reads as 0, and fmaf(w, 0, v) = v
+	const int4* sidx = reinterpret_cast<const int4*>(P.simap_idx) + (P.simap_per_sa ? (size_t)isa * npix : 0);
+	const float4* swt = reinterpret_cast<const float4*>(P.simap_wt) + (P.simap_per_sa ? (size_t)isa * npix : 0);
 	float pix[NPQ];
 #pragma unroll
 	for (int q = 0; q < NPQ; q++) {
 		const int p = lane + 32 * q;
 		float v = 0.f;
 		if (p < npix) {
-#pragma unroll
-			for (int c = 0; c < 4; c++) {
-				const int id = __ldg(sidx + 4 * p + c);
-				if (id >= 0) v = fmaf(__ldg(swt + 4 * p + c), psf[id], v);
-			}
+			const int4 id = __ldg(sidx + p);
+			const float4 w = __ldg(swt + p);
+			v = fmaf(w.x, id.x >= 0 ? psf[id.x] : 0.f, v);
+			v = fmaf(w.y, id.y >= 0 ? psf[id.y] : 0.f, v);
+			v = fmaf(w.z, id.z >= 0 ? psf[id.z] : 0.f, v);
+			v = fmaf(w.w, id.w >= 0 ? psf[id.w] : 0.f, v);
 			v *= W.alpha;
 			if (P.accum) v += W.ints[(size_t)isa * npix + p];  // dtrat > 1: the frames so far
 		}
@@ -984,7 +988,7 @@ __device__ __forceinline__ void r2c32_post(const float2 (&z)[16], float2 (&Q)[16
 		const float2 a = z[K], b = make_float2(z[16 - K].x, -z[16 - K].y);
 		const float2 sm = cadd(a, b), df = csub(a, b);
 		const float2 t = twmul<-1, 32, K>(make_float2(df.y, -df.x));  // w^K * (-i) * (a - b)
-		Q[K] = make_float2(0.5f * (sm.x + t.x), 0.5f * (sm.y + t.y));
+		Q[K] = mul2(make_float2(0.5f, 0.5f), cadd(sm, t));
 		r2c32_post<K + 1>(z, Q);
 	}
 }
@@ -1107,8 +1111,14 @@ __device__ __forceinline__ void otf_tf_inverse_half_n32(const PowfsDev& P, const
 		const float2 g = scr[lane], m = scr[(32 - lane) & 31];
 		float2 y0[1] = {make_float2(0.5f * (g.x + m.x), 0.5f * (g.y - m.y))};
 		float2 y16[1] = {make_float2(0.5f * (g.y + m.y), -0.5f * (g.x - m.x))};
-		tf_apply<1>(P, W, isa, lane * 32, 0, y0);
-		tf_apply<1>(P, W, isa, lane * 32 + 16, 0, y16);
+		// fx and -fx share a read: TF(-fx) = conj TF(fx) on the lines fy = 0 and
+		// 16 (a row of 256 bytes each, so a line per lane)
+		const int hf = lane <= 16 ? lane : 32 - lane;
+		const bool conj = lane > 16;
+		if (conj) y0[0].y = -y0[0].y, y16[0].y = -y16[0].y;
+		tf_apply<1>(P, W, isa, hf * 32, 0, y0);
+		tf_apply<1>(P, W, isa, hf * 32 + 16, 0, y16);
+		if (conj) y0[0].y = -y0[0].y, y16[0].y = -y16[0].y;
 		scr2[lane] = make_float2(y0[0].x - y16[0].y, y0[0].y + y16[0].x);
 	}
 	tf_apply<8>(P, W, isa, 8 * h * 32 + c, 32, A);
