@@ -148,8 +148,6 @@ struct shwfs_ctx {
 	cudaGraphExec_t gexec = nullptr;
 	int g_i0 = -1, g_i1 = -1, g_warm = 0;
 	int capturing = 0;
-	DevBuf<const float*> llt_in;
-	DevBuf<float2*> llt_out;
 	DevBuf<int> errflag;                 // bounded device waits record expiry here
 	int* errflag_h = nullptr;            // pinned copy read by the frame syncs
 	int errflag_armed = 0;               // a kernel that can set errflag ran since the last check
@@ -422,8 +420,6 @@ int shwfs_destroy(shwfs_ctx* ctx) {
 	for (auto e : ctx->ev_pool) cudaEventDestroy(e);
 	ctx->wfsdev.free_();
 	ctx->errflag.free_();
-	ctx->llt_in.free_();
-	ctx->llt_out.free_();
 	cudaStreamSynchronize(ctx->aux);
 	cudaEventDestroy(ctx->ev_fork);
 	cudaEventDestroy(ctx->ev_join);
@@ -1680,28 +1676,21 @@ static int launch_uplink(shwfs_ctx* ctx, const std::vector<int>& wlist, const st
 		for (int k = 0; k < nw; k++) lotfs[k] = ctx->wfs[wlist[k]].lotfT.p;
 		return launch_uplink_gen(ctx, p, wlist, lltopd);
 	}
-	std::vector<const float*> in(nw);
-	std::vector<float2*> out(nw);
-	for (int k = 0; k < nw; k++) {
-		in[k] = lltopd[k];
-		out[k] = ctx->wfs[wlist[k]].lotfT.p;
-		lotfs[k] = out[k];
-	}
-	CK(cudaStreamSynchronize(ctx->stream));
-	int r;
-	if ((r = dev_alloc(ctx, ctx->llt_in, (size_t)nw))) return r;
-	if ((r = dev_alloc(ctx, ctx->llt_out, (size_t)nw))) return r;
-	CK(cudaMemcpyAsync(ctx->llt_in.p, in.data(), sizeof(float*) * nw, cudaMemcpyHostToDevice, ctx->stream));
-	CK(cudaMemcpyAsync(ctx->llt_out.p, out.data(), sizeof(float2*) * nw, cudaMemcpyHostToDevice, ctx->stream));
-	ctx->h2d_bytes += (sizeof(float*) + sizeof(float2*)) * nw;
 	const float twoinvwvl = (float)(2.0 / p.d.wvl);
 	const float lltnorm = (float)(1.0 / ((double)p.d.llt_nx * p.d.embfac * p.d.llt_nx * p.d.embfac));
-	{
+	for (int k0 = 0; k0 < nw; k0 += SHWFS_MAX_ENTRIES) {
+		UplinkParams U;
+		memset(&U, 0, sizeof(U));
+		const int n = std::min(SHWFS_MAX_ENTRIES, nw - k0);
+		for (int k = 0; k < n; k++) {
+			U.lltopd[k] = lltopd[k0 + k];
+			U.lotfT[k] = ctx->wfs[wlist[k0 + k]].lotfT.p;
+			lotfs[k0 + k] = U.lotfT[k];
+		}
 		StageMark m(ctx, SHWFS_STAGE_UPLINK);
-		uplink_otf_n32_kernel<<<(nw + 3) / 4, 128, 0, ctx->stream>>>(ctx->llt_in.p, p.lltamp.p, ctx->llt_out.p, nw,
-			twoinvwvl, lltnorm);
+		uplink_otf_n32_kernel<<<(n + 3) / 4, 128, 0, ctx->stream>>>(U, p.lltamp.p, n, twoinvwvl, lltnorm);
+		CK(cudaGetLastError());
 	}
-	CK(cudaGetLastError());
 	return 0;
 }
 
@@ -2549,17 +2538,13 @@ int shwfs_wfs_update_mtche(shwfs_ctx* ctx, int iwfs, int mtchcr) {
 	if (!se && d.has_llt && !p.lotf_flat.p) {  // without it: the flat uplink OTF
 		if (!p.lltamp.p) return fail(ctx, SHWFS_ESTATE, "update_mtche: LLT amplitude not set");
 		if ((r = dev_alloc(ctx, p.lotf_flat, (size_t)d.notf * d.notf))) return r;
-		DevBuf<const float*> in;
-		DevBuf<float2*> out;
-		const float* zi = p.zero_opd.p;
-		float2* zo = p.lotf_flat.p;
-		if ((r = dev_upload(ctx, in, &zi, 1)) || (r = dev_upload(ctx, out, &zo, 1))) return r;
-		uplink_otf_n32_kernel<<<1, 128, 0, ctx->stream>>>(in.p, p.lltamp.p, out.p, 1, 0.f,
+		UplinkParams U;
+		memset(&U, 0, sizeof(U));
+		U.lltopd[0] = p.zero_opd.p;
+		U.lotfT[0] = p.lotf_flat.p;
+		uplink_otf_n32_kernel<<<1, 128, 0, ctx->stream>>>(U, p.lltamp.p, 1, 0.f,
 			(float)(1.0 / ((double)d.llt_nx * d.embfac * d.llt_nx * d.embfac)));
 		CK(cudaGetLastError());
-		CK(cudaStreamSynchronize(ctx->stream));
-		in.free_();
-		out.free_();
 	}
 	if ((r = dev_alloc(ctx, p.mtch_img, (size_t)nsa * 3 * npix)) || (r = dev_alloc(ctx, p.mtch_red, 2))) return r;
 	if (!w->mtche.p && (r = dev_alloc(ctx, w->mtche, (size_t)nsa * 2 * npix))) return r;

@@ -759,17 +759,22 @@ __global__ void __launch_bounds__(256) llt_uplink_kernel(const __grid_constant__
 }
 
 // Uplink OTF from a given LLT OPD (one warp per WFS), for callers that hold
-// the LLT OPD already (shwfs_ints_grad_dev).
-__global__ void uplink_otf_n32_kernel(const float* const* lltopd, const float* lltamp, float2* const* lotfT,
-	int nwfs, float twoinvwvl, float lltnorm) {
+// the LLT OPD already (shwfs_ints_grad_dev).  The pointers travel with the
+// launch: no table in device memory to wait for and copy.
+struct UplinkParams {
+	const float* lltopd[SHWFS_MAX_ENTRIES];
+	float2* lotfT[SHWFS_MAX_ENTRIES];
+};
+__global__ void uplink_otf_n32_kernel(const __grid_constant__ UplinkParams U, const float* lltamp, int nwfs,
+	float twoinvwvl, float lltnorm) {
 	__shared__ float2 tiles[4][32 * LD];
 	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 	const int iw = blockIdx.x * 4 + warp;
 	if (iw >= nwfs) return;
 	float2 F[32];
-	field_fft_n32(lltopd[iw], lltamp, twoinvwvl, tiles[warp], lane, F);
+	field_fft_n32(U.lltopd[iw], lltamp, twoinvwvl, tiles[warp], lane, F);
 	psf_to_otf_n32(F, lltnorm, tiles[warp], lane);
-	float2* out = lotfT[iw];
+	float2* out = U.lotfT[iw];
 #pragma unroll
 	for (int fx = 0; fx < 32; fx++) out[lane + 32 * fx] = F[fx];
 }
