@@ -1263,6 +1263,8 @@ __device__ __forceinline__ void geom_noise(float& gx, float& gy, int isa, int ns
 // sum a o x, sum a o y), imcc = inv(sum a [1 x y]'[1 x y]), x = origx + ix dx.
 // One warp per subaperture, FP64 sums; with nea, geom_noise is added.
 // blockIdx.y is the WFS: one launch serves every WFS of a powfs.
+// 6 WFS of 2820 16x16 pupils: 52 us as six launches, 20.6 as one, 16.8 with a
+// lane's column sums and the reduce-scatter; bound by issue (62 %) and FP64.
 struct ZtiltWfs {
 	const float *opd, *amp, *nea;
 	float* grad;
@@ -1282,24 +1284,71 @@ __global__ void __launch_bounds__(256) ztilt_kernel(const __grid_constant__ Ztil
 	if (isa >= nsa) return;
 	const int np = nopd * nopd;
 	const double ox = origx[isa], oy = origy[isa];
-	double m[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};  // a00 a01 a02 a11 a12 a22 b0 b1 b2
-	for (int ip = lane; ip < np; ip += 32) {
-		const double x = ox + (ip % nopd) * dx, y = oy + (ip / nopd) * dx;
-		const double a = amp[(size_t)isa * np + ip], ao = a * (double)opd[(size_t)isa * np + ip];
-		m[0] += a;
-		m[1] += a * x;
-		m[2] += a * y;
-		m[3] += a * x * x;
-		m[4] += a * x * y;
-		m[5] += a * y * y;
-		m[6] += ao;
-		m[7] += ao * x;
-		m[8] += ao * y;
+	double m[9];  // a00 a01 a02 a11 a12 a22 b0 b1 b2
+	if (nopd == 16 || nopd == 32) {
+		// a lane's points are one column: its x enters once, after the sums
+		const double x = ox + (lane % nopd) * dx;
+		double sa = 0, say = 0, sayy = 0, so = 0, soy = 0;
+#pragma unroll 8
+		for (int ip = lane; ip < np; ip += 32) {
+			const double y = oy + (ip / nopd) * dx;
+			const double a = amp[(size_t)isa * np + ip], ao = a * (double)opd[(size_t)isa * np + ip], ay = a * y;
+			sa += a;
+			say += ay;
+			sayy += ay * y;
+			so += ao;
+			soy += ao * y;
+		}
+		m[0] = sa;
+		m[1] = sa * x;
+		m[2] = say;
+		m[3] = m[1] * x;
+		m[4] = say * x;
+		m[5] = sayy;
+		m[6] = so;
+		m[7] = so * x;
+		m[8] = soy;
+	} else {
+#pragma unroll
+		for (int k = 0; k < 9; k++) m[k] = 0;
+		for (int ip = lane; ip < np; ip += 32) {
+			const double x = ox + (ip % nopd) * dx, y = oy + (ip / nopd) * dx;
+			const double a = amp[(size_t)isa * np + ip], ao = a * (double)opd[(size_t)isa * np + ip];
+			m[0] += a;
+			m[1] += a * x;
+			m[2] += a * y;
+			m[3] += a * x * x;
+			m[4] += a * x * y;
+			m[5] += a * y * y;
+			m[6] += ao;
+			m[7] += ao * x;
+			m[8] += ao * y;
+		}
 	}
+	// sums over the warp: the first eight as a reduce-scatter (lane k mod 8 ends
+	// with m[k]: nine exchanges instead of forty), then gathered
+	{
+		double v[8];
 #pragma unroll
-	for (int k = 0; k < 9; k++)
+		for (int k = 0; k < 8; k++) v[k] = m[k];
 #pragma unroll
-		for (int off = 16; off > 0; off >>= 1) m[k] += __shfl_xor_sync(0xffffffffu, m[k], off);
+		for (int h = 4; h >= 1; h >>= 1) {
+			const bool up = (lane & h) != 0;
+#pragma unroll
+			for (int k = 0; k < 4; k++) {
+				if (k < h) {
+					const double give = up ? v[k] : v[k + h], keep = up ? v[k + h] : v[k];
+					v[k] = keep + __shfl_xor_sync(0xffffffffu, give, h);
+				}
+			}
+		}
+		v[0] += __shfl_xor_sync(0xffffffffu, v[0], 8);
+		v[0] += __shfl_xor_sync(0xffffffffu, v[0], 16);
+#pragma unroll
+		for (int k = 0; k < 8; k++) m[k] = __shfl_sync(0xffffffffu, v[0], k);
+#pragma unroll
+		for (int off = 16; off > 0; off >>= 1) m[8] += __shfl_xor_sync(0xffffffffu, m[8], off);
+	}
 	if (lane == 0) {
 		const double a00 = m[0], a01 = m[1], a02 = m[2], a11 = m[3], a12 = m[4], a22 = m[5];
 		// inverse of the symmetric 3x3 by cofactors
