@@ -430,14 +430,17 @@ __device__ __forceinline__ void dft8_mid(float2 (&a)[8], float dir) {
 	float2 b[8] = {a[4], a[5], a[2], a[3], make_float2(-a[4].x, -a[4].y), make_float2(-a[5].x, -a[5].y), a[2], a[3]};
 	dft8_tail(b, a, dir);
 }
-// a[i] *= exp(DIR 2 pi i t i / 64); tw[k] = exp(-2 pi i k / 64)
+// a[i] *= exp(DIR 2 pi i t i / 64); tw[N64_TS t + i] = exp(-2 pi i t i / 64), read in pairs
+// (rows 80 bytes apart, so that the rows of a quarter warp fall on distinct banks)
+constexpr int N64_TS = 10;
 template <int DIR>
 __device__ __forceinline__ void n64_twiddle(float2 (&a)[8], const float2* tw, int t) {
+	const float4* w4 = reinterpret_cast<const float4*>(tw + N64_TS * t);
 #pragma unroll
-	for (int i = 1; i < 8; i++) {
-		float2 w = tw[t * i];
-		if (DIR > 0) w.y = -w.y;
-		a[i] = make_float2(a[i].x * w.x - a[i].y * w.y, a[i].x * w.y + a[i].y * w.x);
+	for (int q = 0; q < 4; q++) {
+		const float4 w = w4[q];
+		if (q) a[2 * q] = DIR > 0 ? cmulc(a[2 * q], make_float2(w.x, w.y)) : cmul(a[2 * q], make_float2(w.x, w.y));
+		a[2 * q + 1] = DIR > 0 ? cmulc(a[2 * q + 1], make_float2(w.z, w.w)) : cmul(a[2 * q + 1], make_float2(w.z, w.w));
 	}
 }
 // elements at p[es (8 t + i)] (group t) or p[es (8 i + t)] (stride t) of a line
@@ -470,10 +473,10 @@ __device__ __forceinline__ void n64_put(float2* p, const float2 (&a)[8]) {
 // conflicts (line stride 65) and a warp shares its twiddles; the pass with the
 // transfer functions takes 8 consecutive frequencies of 4 columns 8 apart
 // instead, so that they are read in 64-byte runs.  Against the 16-pass form
-// with 256 threads (6725 -> 4444 wavefronts an image): 6 WFS of 2820 images
-// 464 -> 342 us, 3 WFS of 808 images 71 -> 54 us.
+// with 256 threads (6725 -> 4425 wavefronts an image): 6 WFS of 2820 images
+// 464 -> 334 us, 3 WFS of 808 images 71 -> 52 us.
 constexpr int N64_THREADS = 128;
-constexpr int N64_SMEM_BYTES = (64 * N64_LS + 64) * 8 + 256 * 4;
+constexpr int N64_SMEM_BYTES = (64 * N64_LS + 8 * N64_TS) * 8 + 256 * 4;
 // NOPD > 0 fixes the pupil size at compile time (nopd is then ignored).
 template <int NOPD>
 __global__ void __launch_bounds__(N64_THREADS, 6) ints_n64_kernel(PowfsDev P, const WfsDev* __restrict__ wfs, int nw,
@@ -481,16 +484,16 @@ __global__ void __launch_bounds__(N64_THREADS, 6) ints_n64_kernel(PowfsDev P, co
 	static_assert(NOPD == 0 || NOPD == 32, "fixed pupil sizes: 32");
 	constexpr int LS = N64_LS;
 	const int nopd = NOPD > 0 ? NOPD : nopd_rt;
-	extern __shared__ float2 n64_s[];
+	extern __shared__ __align__(16) float2 n64_s[];
 	float2* img = n64_s;
 	float2* tw = n64_s + 64 * LS;
-	float* spix = reinterpret_cast<float*>(tw + 64);
+	float* spix = reinterpret_cast<float*>(tw + 8 * N64_TS);
 	const int item = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	if (item >= nitem) return;
 	const int isa = item / nw;
 	const WfsDev& W = wfs[item % nw];
 	const int pad = (64 - nopd) / 2, no2 = nopd * nopd;
-	if (tid < 64) tw[tid] = tw64[tid];
+	if (tid < 64) tw[N64_TS * (tid >> 3) + (tid & 7)] = tw64[(tid >> 3) * (tid & 7)];
 	__syncthreads();
 	float2 a[8], b[8];
 	// (b) field, zero-padded (cembed_wvf, maos/wfsints.c:233), and (c) PSF: forward along x on the pupil rows
