@@ -1429,7 +1429,7 @@ static int push_wfsdev(shwfs_ctx* ctx, const std::vector<WfsDev>& wd, const WfsD
 template <int N>
 static int launch_gen_n(shwfs_ctx* ctx, PowfsState& p, GenParams& G) {
 	constexpr int L = gen_lines(N);
-	const size_t smem = ((size_t)L * (N + 1) + N / 2) * sizeof(float2);
+	const size_t smem = gen_tile_smem(N);
 	const dim3 full(G.nitem, N / L), field(G.nitem, (G.nopd + L - 1) / L);
 	gen_pass_kernel<N, GEN_FIELD_COLS><<<field, GEN_THREADS, smem, ctx->stream>>>(G);
 	gen_pass_kernel<N, GEN_PSF_ROWS><<<full, GEN_THREADS, smem, ctx->stream>>>(G);
@@ -1444,7 +1444,7 @@ static int launch_gen_n(shwfs_ctx* ctx, PowfsState& p, GenParams& G) {
 static int ensure_twiddles(shwfs_ctx* ctx, PowfsState& p) {
 	if (p.gen_tw.p) return 0;
 	const int N = p.d.notf;
-	std::vector<float2> tw(N);  // the passes use the first N/2, the fused 64-point kernel all N
+	std::vector<float2> tw(N);  // exp(-2 pi i k / N)
 	for (int k = 0; k < N; k++) tw[k] = make_float2((float)cos(2 * M_PI * k / N), (float)-sin(2 * M_PI * k / N));
 	return dev_upload(ctx, p.gen_tw, tw.data(), tw.size());
 }
@@ -2292,9 +2292,9 @@ static int frame_worklist(shwfs_ctx* ctx, const std::vector<std::vector<int>>& w
 	static int resident[64][6] = {{0}};
 	if (ctx->device >= 64) return fail(ctx, SHWFS_EINVAL, "work list: device %d out of range", ctx->device);
 	if (!resident[ctx->device][kv]) {
-		CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WL_N32_SMEM));
+		CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WL_SMEM));
 		int per_sm = 0, nsm = 0;
-		CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, WL_THREADS, WL_N32_SMEM));
+		CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, WL_THREADS, WL_SMEM));
 		CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
 		resident[ctx->device][kv] = std::max(1, per_sm) * nsm;
 	}
@@ -2303,7 +2303,7 @@ static int frame_worklist(shwfs_ctx* ctx, const std::vector<std::vector<int>>& w
 	const int grid = std::min(W.nwork, resident[ctx->device][kv]);
 	{
 		StageMark mark(ctx, SHWFS_STAGE_INTS);
-		kern<<<grid, WL_THREADS, WL_N32_SMEM, ctx->stream>>>(W);
+		kern<<<grid, WL_THREADS, WL_SMEM, ctx->stream>>>(W);
 		ctx->errflag_armed = 1;
 	}
 	CK(cudaGetLastError());

@@ -1,9 +1,8 @@
 // Imaging stages (b)-(e) for the larger FFT sizes, n_f = n_w = N in {64, 128,
 // 256} (the NGS and tip-tilt sensors of an uneven batch, large-sampling LGS):
 // a chain of batched 1-D FFT passes over a per-powfs scratch image in global
-// memory (L2-resident for the small batches), each pass a kernel that moves
-// tiles of 16 rows or 16 columns of an image through shared memory, with the
-// element-wise step of the chain fused in:
+// memory (L2-resident for the small batches), each pass a kernel over tiles of
+// rows or columns of an image, with the element-wise step of the chain fused in:
 //
 //   pass 1  columns x in [pad, pad+n_o): field E = amp exp(i 2 pi opd / lambda), FFT along y
 //   pass 2  rows ky:                     FFT along x (columns outside the pupil are zero),
@@ -30,81 +29,58 @@
 
 namespace shwfs {
 
-// FFT lines per tile: 16 (128-byte row segments in the column passes), fewer
-// for the large transforms of the small batches, for more blocks
-__host__ __device__ constexpr int gen_lines(int n) { return n >= 256 ? 4 : n >= 128 ? 8 : 16; }
-constexpr int GEN_THREADS = 256;
+// FFT lines per tile: what GEN_THREADS threads of 16 points hold
+__host__ __device__ constexpr int gen_lines(int n) { return 2048 / n; }
+constexpr int GEN_THREADS = 128;
 
 enum GenPass { GEN_FIELD_COLS = 1, GEN_PSF_ROWS, GEN_OTF_COLS, GEN_INV_ROWS };
 constexpr int GEN_NPASS = 4;
 
-__host__ __device__ constexpr int ilog2c(int n) { return n <= 1 ? 0 : 1 + ilog2c(n / 2); }
-
-// Radix-2 decimation-in-time butterfly: (u, v) -> (u + w v, u - w v).
-__device__ __forceinline__ void gen_bfly(float2& u, float2& v, float2 w) {
-	const float2 t = make_float2(v.x * w.x - v.y * w.y, v.x * w.y + v.y * w.x);
-	v = make_float2(u.x - t.x, u.y - t.y);
-	u = make_float2(u.x + t.x, u.y + t.y);
+// Line stride of a tile in the exchange (float2): the 16 (N / 16 + 1) slots of a
+// line, padded so that the lanes of a half warp fall on distinct banks where
+// they run along the lines' elements (row passes) or across the lines.
+__host__ __device__ constexpr int gen_ls(int n, bool rows) {
+	return n == 64 ? (rows ? 84 : 81) : n == 128 ? (rows ? 152 : 153) : (rows ? 272 : 274);
 }
 
-// In-place FFT of gen_lines(N) lines of N points in shared memory, line stride
-// N + 1 (bank-conflict free for column tiles), input in bit-reversed order.
-// tw[k] = exp(-2 pi i k / N), k < N/2; dir -1 forward, +1 inverse.  The
-// log2 N radix-2 stages run two at a time: a thread takes the four points
-// k0 + {0, h, 2h, 3h} (h = 2^st) and applies stage st's butterflies (k0, k0+h)
-// and (k0+2h, k0+3h), then stage st+1's (k0, k0+2h) and (k0+h, k0+3h), with
-// those stages' twiddles -- every point sees the operations of the stage-by-
-// stage transform in the same order, with half its barriers and shared-memory
-// round trips (an odd log2 N starts with one radix-2 stage).
-template <int N, int NT = GEN_THREADS>
-__device__ __forceinline__ void fft_lines(float2* s, const float2* __restrict__ tw, int dir) {
-	constexpr int LOGN = ilog2c(N), LS = N + 1, NB = gen_lines(N) * N / 2, NQ = gen_lines(N) * N / 4;
-	int st = 0;
-	if (LOGN & 1) {  // stage 0: half = 1, twiddle tw[0]
-		float2 w0 = tw[0];
-		if (dir > 0) w0.y = -w0.y;
-		for (int b = threadIdx.x; b < NB; b += NT) {
-			const int line = b / (N / 2), j = b - line * (N / 2);
-			float2* a = s + line * LS + 2 * j;
-			float2 u = a[0], v = a[1];
-			gen_bfly(u, v, w0);
-			a[0] = u;
-			a[1] = v;
-		}
-		__syncthreads();
-		st = 1;
+// FFT of a line of N points by its T = N / 16 threads of 16 points each:
+// thread t brings v[i] = x[T i + t] and leaves with v[i] = X[t + T i] (natural
+// order, unnormalised; DIR -1 forward, +1 inverse).  A 16-point transform in
+// registers, the twiddles w_N^(t k1), one exchange through the line's slots
+// ex[k1 (T + 1) + t], then the 16 / T T-point transforms of k1 = t + T m:
+//   X[k1 + 16 k2] = sum_t w_T^(t k2) w_N^(t k1) sum_i w_16^(i k1) x[T i + t].
+// The outputs sit where the next transform of the line takes its inputs, so a
+// pass that transforms its lines twice stays in registers in between: one
+// shared-memory round trip a transform, where radix-2 stages taken two at a
+// time made four with a block barrier each.  52 images of 128 x 128 points, the
+// four passes one after the other with cold caches: 8 + 17 + 18 + 11 -> 8 + 6 +
+// 13 + 8 us; images and gradients in one call 39 -> 19 us (its five launches now
+// set the rate).  ROWS: a line's threads are lanes of one warp.
+// tw[k] = exp(-2 pi i k / N), k < N.
+template <int N, int DIR, bool ROWS>
+__device__ __forceinline__ void gen_fft(float2 (&v)[16], float2* ex, int t, const float2* __restrict__ tw) {
+	constexpr int T = N / 16, M = 16 / T;
+	fft_reg<DIR, 16>(v);
+#pragma unroll
+	for (int k = 1; k < 16; k++) {
+		const float2 w = __ldg(tw + t * k);
+		v[k] = DIR > 0 ? cmulc(v[k], w) : cmul(v[k], w);
 	}
-#pragma unroll 1
-	for (; st < LOGN; st += 2) {
-		const int h = 1 << st;
-		for (int b = threadIdx.x; b < NQ; b += NT) {
-			const int line = b / (N / 4), j = b - line * (N / 4);
-			const int grp = j >> st, pos = j & (h - 1);
-			float2* a = s + line * LS + grp * 4 * h + pos;
-			float2 w1 = tw[pos << (LOGN - 1 - st)];
-			float2 w2 = tw[pos << (LOGN - 2 - st)], w3 = tw[(pos + h) << (LOGN - 2 - st)];
-			if (dir > 0) {
-				w1.y = -w1.y;
-				w2.y = -w2.y;
-				w3.y = -w3.y;
-			}
-			float2 x0 = a[0], x1 = a[h], x2 = a[2 * h], x3 = a[3 * h];
-			gen_bfly(x0, x1, w1);  // stage st
-			gen_bfly(x2, x3, w1);
-			gen_bfly(x0, x2, w2);  // stage st + 1
-			gen_bfly(x1, x3, w3);
-			a[0] = x0;
-			a[h] = x1;
-			a[2 * h] = x2;
-			a[3 * h] = x3;
-		}
-		__syncthreads();
+#pragma unroll
+	for (int k = 0; k < 16; k++) ex[k * (T + 1) + t] = v[k];
+	if (ROWS) __syncwarp();
+	else __syncthreads();
+#pragma unroll
+	for (int m = 0; m < M; m++) {
+		float2 u[T];
+#pragma unroll
+		for (int j = 0; j < T; j++) u[j] = ex[(t + T * m) * (T + 1) + j];
+		fft_reg<DIR, T>(u);
+#pragma unroll
+		for (int k2 = 0; k2 < T; k2++) v[m + M * k2] = u[k2];
 	}
-}
-
-template <int N>
-__device__ __forceinline__ int bitrev(int k) {
-	return (int)(__brev((unsigned)k) >> (32 - ilog2c(N)));
+	if (ROWS) __syncwarp();  // the slots may be written again
+	else __syncthreads();
 }
 
 // A launch covers nitem images.  WFS mode: image i is subaperture i / nw of
@@ -117,7 +93,7 @@ struct GenParams {
 	float scale;                 // factor on |.|^2: 1 for WFS images, 1/N^2 for LLT pupils
 	float twoinvwvl;
 	float2* buf;                 // nitem * N * N scratch, row-major per image
-	const float2* tw;            // N/2 twiddles exp(-2 pi i k / N)
+	const float2* tw;            // N twiddles exp(-2 pi i k / N)
 	const WfsDev* wfs;
 	const float2* etfT1;         // nsa * N^2 transposed, or null
 	const float2* etfT2;
@@ -126,8 +102,12 @@ struct GenParams {
 	int nominal_per_sa;
 };
 
-// Shared memory of one pass tile: the lines (stride N + 1) and N/2 twiddles.
-__host__ __device__ constexpr int gen_tile_smem(int n) { return (gen_lines(n) * (n + 1) + n / 2) * (int)sizeof(float2); }
+// Shared memory of one pass tile: the exchange, and the tile's transfer
+// functions (or uplink OTF) by line and frequency (line stride N + 1).
+__host__ __device__ constexpr int gen_tile_smem(int n) {
+	return gen_lines(n) * ((gen_ls(n, true) > gen_ls(n, false) ? gen_ls(n, true) : gen_ls(n, false)) + n + 1) *
+		(int)sizeof(float2);
+}
 
 // Reads of the scratch image: through L1, or from L2 only (L2ONLY) where other
 // blocks of the same launch wrote it (L1 is not coherent between SMs).
@@ -137,124 +117,116 @@ __device__ __forceinline__ float2 gen_ld(const float2* p) {
 	else return *p;
 }
 
-// Element-wise step f(value, line, k) over a tile's lines in natural order,
-// the results left in bit-reversed order along each line for the line's next
-// transform (a pass that transforms its lines twice).
-template <int N, int NT, typename F>
-__device__ __forceinline__ void gen_permute(float2* s, F f) {
-	constexpr int LS = N + 1, NE = gen_lines(N) * N / NT;
-	static_assert(gen_lines(N) * N % NT == 0, "tile elements per thread");
-	float2 v[NE];
-#pragma unroll
-	for (int e = 0; e < NE; e++) {
-		const int idx = threadIdx.x + e * NT, line = idx / N, k = idx - line * N;
-		v[e] = f(s[line * LS + k], line, k);
-	}
-	__syncthreads();
-#pragma unroll
-	for (int e = 0; e < NE; e++) {
-		const int idx = threadIdx.x + e * NT, line = idx / N, k = idx - line * N;
-		s[line * LS + bitrev<N>(k)] = v[e];
-	}
-	__syncthreads();
-}
-
-// One pass over tile `tile` of image i by a block of NT threads; gen_s is the
-// tile's shared memory (gen_tile_smem(N) bytes).
+// One pass over tile `tile` of image i by a block of GEN_THREADS threads; gen_s
+// is the tile's shared memory (gen_tile_smem(N) bytes).  The scratch image
+// goes straight between global memory and registers: consecutive lanes take
+// consecutive elements of a row, or consecutive columns.
 template <int N, int PASS, int NT, bool L2ONLY>
 __device__ __forceinline__ void gen_pass_tile(const GenParams& G, int i, int tile, float2* gen_s) {
-	constexpr int LS = N + 1, GEN_LINES = gen_lines(N);
+	constexpr int L = gen_lines(N), T = N / 16;
 	constexpr bool ROWS = PASS == GEN_PSF_ROWS || PASS == GEN_INV_ROWS;
-	float2* tw = gen_s + GEN_LINES * LS;  // N/2 twiddles
+	constexpr int LS = gen_ls(N, ROWS), TLS = N + 1;
+	static_assert(NT == L * T && NT == GEN_THREADS, "a thread per 16 points of the tile");
 	const int isa = G.uplink ? 0 : i / G.nw;
 	const WfsDev& W = G.wfs[G.uplink ? i : i % G.nw];
 	float2* im = G.buf + (size_t)i * N * N;
 	const int tid = threadIdx.x;
-	for (int k = tid; k < N / 2; k += NT) tw[k] = G.tw[k];
-	int l0 = tile * GEN_LINES, nl = GEN_LINES;  // first line and lines of the tile
+	const int line = ROWS ? tid / T : tid % L, t = ROWS ? tid % T : tid / L;
+	float2* ex = gen_s + line * LS;
+	float2* tfs = gen_s + L * (gen_ls(N, true) > gen_ls(N, false) ? gen_ls(N, true) : gen_ls(N, false));
+	int l0 = tile * L, nl = L;  // first line and lines of the tile
 	if (PASS == GEN_FIELD_COLS) {  // only the pupil's columns
-		nl = min(GEN_LINES, G.nopd - l0);
+		nl = min(L, G.nopd - l0);
 		l0 += G.pad;
 	}
-	// ---- load (bit-reversed along the line)
-	for (int idx = tid; idx < GEN_LINES * N; idx += NT) {
-		int line, k;
-		if (ROWS) {
-			line = idx / N;
-			k = idx - line * N;
-		} else {
-			k = idx / GEN_LINES;
-			line = idx - k * GEN_LINES;
+	const size_t at0 = ROWS ? (size_t)(l0 + line) * N + t : (size_t)t * N + l0 + line;
+	constexpr size_t STEP = ROWS ? T : (size_t)T * N;
+	float2 v[16];
+	if (PASS == GEN_FIELD_COLS) {
+		float o[16], a[16];
+		const int x = l0 + line - G.pad;
+#pragma unroll
+		for (int k = 0; k < 16; k++) {
+			const int y = T * k + t - G.pad;
+			const bool in = line < nl && y >= 0 && y < G.nopd;
+			const size_t e = (size_t)isa * G.nopd * G.nopd + (size_t)y * G.nopd + x;
+			o[k] = in ? __ldg(W.opd + e) : 0.f;
+			a[k] = in ? __ldg(W.amp + e) : 0.f;
 		}
-		float2 v = make_float2(0.f, 0.f);
-		if (line < nl) {
-			if (PASS == GEN_FIELD_COLS) {
-				const int x = l0 + line - G.pad, y = k - G.pad;
-				if (y >= 0 && y < G.nopd) {
-					const size_t e = (size_t)isa * G.nopd * G.nopd + (size_t)y * G.nopd + x;
-					const float o = __ldg(W.opd + e), a = __ldg(W.amp + e);
-					float sn, cs;
-					sincospif(G.twoinvwvl * o, &sn, &cs);
-					v = make_float2(a * cs, a * sn);
-				}
-			} else if (!ROWS) {
-				v = gen_ld<L2ONLY>(im + (size_t)k * N + l0 + line);
-			} else if (PASS != GEN_PSF_ROWS || (k >= G.pad && k < G.pad + G.nopd)) {
-				v = gen_ld<L2ONLY>(im + (size_t)(l0 + line) * N + k);  // columns outside the pupil are zero
+#pragma unroll
+		for (int k = 0; k < 16; k++) {
+			const int y = T * k + t - G.pad;
+			v[k] = make_float2(0.f, 0.f);
+			if (line < nl && y >= 0 && y < G.nopd) {
+				float sn, cs;
+				sincospif(G.twoinvwvl * o[k], &sn, &cs);
+				v[k] = make_float2(a[k] * cs, a[k] * sn);
 			}
 		}
-		gen_s[line * LS + bitrev<N>(k)] = v;
+	} else {
+#pragma unroll
+		for (int k = 0; k < 16; k++) {
+			const int n = T * k + t;  // rows of pass 2: columns outside the pupil are zero
+			v[k] = PASS != GEN_PSF_ROWS || (n >= G.pad && n < G.pad + G.nopd) ? gen_ld<L2ONLY>(im + at0 + STEP * k)
+																				: make_float2(0.f, 0.f);
+		}
 	}
-	__syncthreads();
-	fft_lines<N, NT>(gen_s, tw, PASS == GEN_INV_ROWS ? 1 : -1);
+	if (PASS == GEN_OTF_COLS && !G.uplink) {
+		// the tile's transfer functions ([fy + N fx], fy fastest) in runs of fy: conj(uplink OTF) x ETF / nominal
+		const size_t f0 = (size_t)N * l0;
+		const float2* e1 = G.etfT1 ? G.etfT1 + (size_t)isa * N * N + f0 : nullptr;
+		const float2* e2 = G.etfT2 ? G.etfT2 + (size_t)isa * N * N + f0 : nullptr;
+		const float* nm = G.nominalT ? G.nominalT + (G.nominal_per_sa ? (size_t)isa * N * N : 0) + f0 : nullptr;
+		const float2* up = W.lotfT ? W.lotfT + f0 : nullptr;
+#pragma unroll 4
+		for (int k = 0; k < 16; k++) {
+			const int idx = tid + k * NT;
+			float2 w = make_float2(1.f, 0.f);
+			if (e1) {
+				w = __ldg(e1 + idx);
+				if (e2) {
+					const float2 b = __ldg(e2 + idx);
+					w = make_float2(w.x * G.etfwt1 + b.x * G.etfwt2, w.y * G.etfwt1 + b.y * G.etfwt2);
+				}
+			} else if (nm) {
+				w.x = __ldg(nm + idx);
+			}
+			if (up) w = cmulc(w, __ldg(up + idx));
+			tfs[(idx / N) * TLS + idx % N] = w;
+		}
+	}
+	gen_fft<N, PASS == GEN_INV_ROWS ? 1 : -1, ROWS>(v, ex, t, G.tw);
 	// ---- element-wise steps of the chain, and a pass's second transform
 	if (PASS == GEN_PSF_ROWS) {
 		// |.|^2 * scale: the PSF row, then its own transform along x (the OTF's)
-		gen_permute<N, NT>(gen_s, [&](float2 v, int, int) { return make_float2((v.x * v.x + v.y * v.y) * G.scale, 0.f); });
-		fft_lines<N, NT>(gen_s, tw, -1);
+#pragma unroll
+		for (int k = 0; k < 16; k++) v[k] = make_float2((v[k].x * v[k].x + v[k].y * v[k].y) * G.scale, 0.f);
+		gen_fft<N, -1, ROWS>(v, ex, t, G.tw);
 	}
 	if (PASS == GEN_OTF_COLS) {
-		// line = fx - l0, element fy: the OTF; transfer functions are [fy + N fx], fy fastest
+		// line = fx - l0, element fy = t + T k: the OTF
 		if (G.uplink) {
-			for (int idx = tid; idx < GEN_LINES * N; idx += NT) {
-				const int line = idx / N, fy = idx - line * N;
-				const_cast<float2*>(W.lotfT)[(size_t)fy + (size_t)N * (l0 + line)] = gen_s[line * LS + fy];  // the uplink OTF
+#pragma unroll
+			for (int k = 0; k < 16; k++) tfs[line * TLS + t + T * k] = v[k];
+			__syncthreads();
+#pragma unroll 4
+			for (int k = 0; k < 16; k++) {
+				const int idx = tid + k * NT;
+				const_cast<float2*>(W.lotfT)[(size_t)N * l0 + idx] = tfs[(idx / N) * TLS + idx % N];  // the uplink OTF
 			}
 			return;
 		}
-		gen_permute<N, NT>(gen_s, [&](float2 v, int line, int fy) {
-			const size_t t = (size_t)fy + (size_t)N * (l0 + line);
-			if (W.lotfT) v = cmulc(v, __ldg(W.lotfT + t));
-			if (G.etfT1) {
-				float2 e = __ldg(G.etfT1 + (size_t)isa * N * N + t);
-				if (G.etfT2) {
-					const float2 e2 = __ldg(G.etfT2 + (size_t)isa * N * N + t);
-					e = make_float2(e.x * G.etfwt1 + e2.x * G.etfwt2, e.y * G.etfwt1 + e2.y * G.etfwt2);
-				}
-				v = cmul(v, e);
-			} else if (G.nominalT) {
-				const float d = __ldg(G.nominalT + (G.nominal_per_sa ? (size_t)isa * N * N : 0) + t);
-				v = make_float2(v.x * d, v.y * d);
-			}
-			return v;
-		});
-		fft_lines<N, NT>(gen_s, tw, 1);  // the inverse along fy
+		// gen_fft's barriers lie between the stores to tfs and these reads
+#pragma unroll
+		for (int k = 0; k < 16; k++) v[k] = cmul(v[k], tfs[line * TLS + t + T * k]);
+		gen_fft<N, 1, ROWS>(v, ex, t, G.tw);  // the inverse along fy
 	}
 	// ---- store (natural order; the last pass keeps the real part)
-	for (int idx = tid; idx < GEN_LINES * N; idx += NT) {
-		int line, k;
-		if (ROWS) {
-			line = idx / N;
-			k = idx - line * N;
-		} else {
-			k = idx / GEN_LINES;
-			line = idx - k * GEN_LINES;
-		}
-		if (line < nl) {
-			float2 v = gen_s[line * LS + k];
-			if (PASS == GEN_INV_ROWS) v.y = 0.f;
-			if (ROWS) im[(size_t)(l0 + line) * N + k] = v;
-			else im[(size_t)k * N + l0 + line] = v;
+	if (line < nl) {
+#pragma unroll
+		for (int k = 0; k < 16; k++) {
+			if (PASS == GEN_INV_ROWS) v[k].y = 0.f;
+			im[at0 + STEP * k] = v[k];
 		}
 	}
 }

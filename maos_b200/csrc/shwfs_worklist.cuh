@@ -36,7 +36,8 @@ enum WorkType { WL_N32 = 0, WL_TILE = 1, WL_PIX = 2 };
 constexpr int WL_THREADS = 128;
 constexpr int WL_MAX_SEG = 4;
 constexpr long long WL_WAIT_CYCLES = 4000000000LL;  // ~2 s at 1.9 GHz
-constexpr int WL_N32_SMEM = 4 * 32 * LD * (int)sizeof(float2);
+constexpr int wl_max(int a, int b) { return a > b ? a : b; }
+constexpr int WL_SMEM = wl_max(4 * 32 * LD * (int)sizeof(float2), wl_max(gen_tile_smem(128), gen_tile_smem(256)));
 
 // One powfs of the frame.
 struct WorkSeg {

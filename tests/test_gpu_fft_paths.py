@@ -1,8 +1,11 @@
-"""Imaging at FFT 64 and the cropped science PSF against plain FP64 transforms.
+"""Imaging at FFT 64, 128 and 256 and the cropped science PSF against plain
+FP64 transforms.
 
 FFT 64 (ints_n64_kernel): pupils of 16, 32 and 64 points (the fixed size and
-the general one), a DTF nominal or an ETF with an uplink OTF, and pixel counts
-below, at and above a block's threads.  Tolerance: noise-free intensities
+the general one), a DTF nominal or an ETF with an uplink OTF (which the FFT
+passes form at 64 points), and pixel counts below, at and above a block's
+threads.  FFT 128 and 256 (the FFT passes): pupils that fill their last tile of
+columns and pupils that do not.  Tolerance: noise-free intensities
 within 1e-5 of the subaperture total, the bar of the other imaging tests.
 
 Science PSF: crops of at most 256 pixels run the two-pass transforms
@@ -28,13 +31,14 @@ def _kernel_tf(rng, shape, N):
     return np.fft.fft2(k / 9)
 
 
-@pytest.mark.parametrize("nopd,pix", [(32, 5), (32, 12), (32, 16), (16, 8), (64, 11)])
+@pytest.mark.parametrize("N,nopd,pix", [(64, 32, 5), (64, 32, 12), (64, 32, 16), (64, 16, 8), (64, 64, 11),
+                                        (128, 64, 16), (128, 8, 7), (256, 128, 9), (256, 4, 16)])
 @pytest.mark.parametrize("lgs", [False, True])
-def test_fft64_images_match_plain(nopd, pix, lgs):
+def test_images_match_plain(N, nopd, pix, lgs):
     import torch
     from maos_b200 import shwfs
     rng = np.random.default_rng(nopd * 100 + pix)
-    N, nsa, nllt, wvl = 64, 5, nopd, 0.6e-6  # an LLT pupil has the subapertures' sampling
+    nsa, nllt, wvl = 5, nopd, 0.6e-6  # an LLT pupil has the subapertures' sampling
     npix = pix * pix
     ctx = shwfs.Context(0)
     ip = ctx.powfs_add(nsa=nsa, nopd=nopd, embfac=N // nopd, notf=N, pixpsax=pix, pixpsay=pix, pixthetax=1e-6,
