@@ -2046,32 +2046,44 @@ static int trace_powfs(shwfs_ctx* ctx, int ip, const std::vector<int>& wl, int i
 		}
 	}
 	const int per = p.d.has_llt ? SHWFS_MAX_ENTRIES / (2 + (p.d.notf == 32 ? nb : 0)) : SHWFS_MAX_ENTRIES;
+	const bool gen_llt = p.d.has_llt && p.d.notf != 32;  // uplink OTFs by the FFT passes
 	for (size_t b = 0; b < wl.size(); b += per) {
-		GeomParams gp;
+		GeomParams gp, lp;
 		geom_init(ctx, gp);
+		if (gen_llt) geom_init(ctx, lp);
+		std::vector<int> bw;
+		std::vector<const float*> lo;
 		for (size_t k = b; k < wl.size() && k < b + per; k++) {
 			WfsState& w = ctx->wfs[wl[k]];
 			if ((r = add_wfs_entry(ctx, gp, w, isim, w.opd.p))) return r;
-			if (p.d.has_llt && (r = add_llt_entry(ctx, gp, w, isim))) return r;
+			if (p.d.has_llt && (r = add_llt_entry(ctx, gen_llt ? lp : gp, w, isim))) return r;
 			if (p.d.has_llt && p.d.notf == 32)
 				for (int ib : p.bands)
 					if ((r = add_llt_band_entry(ctx, gp, w, isim, ctx->powfs[ib], ctx->powfs[ib].band_lotf[wl[k]].p)))
 						return r;
+			bw.push_back(wl[k]);
+			lo.push_back(w.lltopd.p);
 		}
+		if (gen_llt) CK(cudaEventRecord(ctx->ev_fork, ctx->stream));
 		if ((r = launch_geom(ctx, gp))) return r;
-		if (p.d.has_llt && p.d.notf != 32) {
-			std::vector<int> bw;
-			std::vector<const float*> lo;
-			for (size_t k = b; k < wl.size() && k < b + per; k++) {
-				bw.push_back(wl[k]);
-				lo.push_back(ctx->wfs[wl[k]].lltopd.p);
-			}
-			if ((r = launch_uplink_gen(ctx, p, bw, lo))) return r;
-			for (int ib : p.bands) {
+		if (gen_llt) {
+			// the LLT pupils' trace and uplink OTFs (a handful of blocks in four dependent
+			// launches: 35 us for the six LGS at FFT 64) on the aux stream beside the
+			// subapertures' trace, as launch_geom does for the 32-point uplink
+			CK(cudaStreamWaitEvent(ctx->aux, ctx->ev_fork, 0));
+			cudaStream_t main = ctx->stream;
+			ctx->stream = ctx->aux;
+			r = launch_geom_wfs(ctx, lp);
+			if (!r) r = launch_uplink_gen(ctx, p, bw, lo);
+			for (size_t j = 0; j < p.bands.size() && !r; j++) {
 				std::vector<float2*> out;
-				for (int i : bw) out.push_back(ctx->powfs[ib].band_lotf[i].p);
-				if ((r = launch_uplink_gen(ctx, ctx->powfs[ib], bw, lo, &out))) return r;
+				for (int i : bw) out.push_back(ctx->powfs[p.bands[j]].band_lotf[i].p);
+				r = launch_uplink_gen(ctx, ctx->powfs[p.bands[j]], bw, lo, &out);
 			}
+			ctx->stream = main;
+			CK(cudaEventRecord(ctx->ev_join, ctx->aux));
+			CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_join, 0));
+			if (r) return r;
 		}
 	}
 	return 0;
