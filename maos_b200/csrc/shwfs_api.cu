@@ -953,7 +953,7 @@ static void geom_init(shwfs_ctx* ctx, GeomParams& gp) {
 }
 
 // LLT pupils go to llt_uplink_kernel on the aux stream (forked from and
-// joined back into the main stream); subaperture pupils to geom_kernel.
+// joined back into the main stream); subaperture pupils to launch_geom_wfs.
 static int launch_geom(shwfs_ctx* ctx, GeomParams& all) {
 	GeomParams gp, lp;
 	memcpy(&gp, &all, sizeof(GeomParams));

@@ -4,7 +4,7 @@
 //
 // The aperture (a regular grid) is held as 16x16 tiles: the tiles that hold
 // aperture points get a slot, and the OPD of a direction is slot-major,
-// 256 points per slot, row-major inside a tile.  geom_kernel traces the
+// 256 points per slot, row-major inside a tile.  geom_rows_kernel traces the
 // tiles like subapertures; points of a tile outside the aperture carry zero
 // amplitude, so every sum below equals the one over the aperture points.
 #pragma once

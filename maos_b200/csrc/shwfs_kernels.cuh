@@ -1,6 +1,6 @@
 // Device kernels of the Shack-Hartmann frame.
 //
-//   geom_kernel         (a) bilinear gather of every turbulence layer into the
+//   geom_rows_kernel    (a) bilinear gather of every turbulence layer into the
 //                           subaperture OPD points of every WFS of the frame
 //                           (FP64 offsets), and the LGS uplink OTF
 //   ints_n32_kernel     (b)-(e) fused per subaperture for n_w = n_f = 32,
@@ -320,7 +320,8 @@ __device__ __forceinline__ void psf_to_otf_n32(float2 (&F)[32], float scale, flo
 }
 
 // ---------------------------------------------------------------------------
-// (a) ray trace of every pupil of the frame in one launch (geom_kernel), and
+// (a) ray trace of every pupil of the frame in one launch (geom_kernel, or
+// geom_rows_kernel for 16x16 and 32x32 pupils), and
 // the LGS uplink OTF of the 32-point path (llt_uplink_kernel): an LLT block
 // keeps its OPD in shared memory and its first warp turns it into
 // lotf = FFT(|FFT(embed(lltamp*exp(i*2*pi*opd/wvl)))|^2 / nlwvf^2), stored
@@ -699,7 +700,7 @@ __global__ void __launch_bounds__(32 * geom_rows_warps(NOPD, ROWS) * geom_rows_p
 
 // LGS uplink: ray trace of each LLT pupil (one block of 256 threads per
 // pupil, nopd == 16) into shared memory, then its first warp forms the
-// uplink OTF.  Runs beside geom_kernel on a second stream.
+// uplink OTF.  Runs beside the subapertures' trace on a second stream.
 __global__ void __launch_bounds__(256) llt_uplink_kernel(const __grid_constant__ GeomParams P) {
 	__shared__ float s_opd[256];
 	__shared__ float2 s_tile[32 * LD];
@@ -925,7 +926,7 @@ __device__ __forceinline__ void ints_n32_pixels(const PowfsDev& P, const WfsDev&
 	// pixel sampling (mkh bilinear map, up to 4 taps per pixel)
 	const int npix = P.npix;
 	// a pixel's 4 map entries are one 16-byte row (cudaMalloc'd, 4 entries per
-	// pixel); a missing tap (index < 0) reads as 0, and fmaf(w, 0, v) = v
+	// pixel); a missing tap (index < 0) is left out, whatever its weight
 	const int4* sidx = reinterpret_cast<const int4*>(P.simap_idx) + (P.simap_per_sa ? (size_t)isa * npix : 0);
 	const float4* swt = reinterpret_cast<const float4*>(P.simap_wt) + (P.simap_per_sa ? (size_t)isa * npix : 0);
 	float pix[NPQ];
@@ -936,10 +937,10 @@ __device__ __forceinline__ void ints_n32_pixels(const PowfsDev& P, const WfsDev&
 		if (p < npix) {
 			const int4 id = __ldg(sidx + p);
 			const float4 w = __ldg(swt + p);
-			v = fmaf(w.x, id.x >= 0 ? psf[id.x] : 0.f, v);
-			v = fmaf(w.y, id.y >= 0 ? psf[id.y] : 0.f, v);
-			v = fmaf(w.z, id.z >= 0 ? psf[id.z] : 0.f, v);
-			v = fmaf(w.w, id.w >= 0 ? psf[id.w] : 0.f, v);
+			if (id.x >= 0) v = fmaf(w.x, psf[id.x], v);
+			if (id.y >= 0) v = fmaf(w.y, psf[id.y], v);
+			if (id.z >= 0) v = fmaf(w.z, psf[id.z], v);
+			if (id.w >= 0) v = fmaf(w.w, psf[id.w], v);
 			v *= W.alpha;
 			if (P.accum) v += W.ints[(size_t)isa * npix + p];  // dtrat > 1: the frames so far
 		}
@@ -1116,14 +1117,8 @@ __device__ __forceinline__ void otf_tf_inverse_half_n32(const PowfsDev& P, const
 		const float2 g = scr[lane], m = scr[(32 - lane) & 31];
 		float2 y0[1] = {make_float2(0.5f * (g.x + m.x), 0.5f * (g.y - m.y))};
 		float2 y16[1] = {make_float2(0.5f * (g.y + m.y), -0.5f * (g.x - m.x))};
-		// fx and -fx share a read: TF(-fx) = conj TF(fx) on the lines fy = 0 and
-		// 16 (a row of 256 bytes each, so a line per lane)
-		const int hf = lane <= 16 ? lane : 32 - lane;
-		const bool conj = lane > 16;
-		if (conj) y0[0].y = -y0[0].y, y16[0].y = -y16[0].y;
-		tf_apply<1>(P, W, isa, hf * 32, 0, y0);
-		tf_apply<1>(P, W, isa, hf * 32 + 16, 0, y16);
-		if (conj) y0[0].y = -y0[0].y, y16[0].y = -y16[0].y;
+		tf_apply<1>(P, W, isa, lane * 32, 0, y0);
+		tf_apply<1>(P, W, isa, lane * 32 + 16, 0, y16);
 		scr2[lane] = make_float2(y0[0].x - y16[0].y, y0[0].y + y16[0].x);
 	}
 	tf_apply<8>(P, W, isa, 8 * h * 32 + c, 32, A);
