@@ -290,10 +290,10 @@ def _roofline(form, cfg, wl, st, units_per_step):
         with open(tp) as f:
             measured = json.load(f)
     traffic = measured.get(f"{cfg['name']}:{form}:ints")
-    raytrace = {"kernel": "geom_kernel", "bound": "hbm", "achieved": ray_gbs, "peak": hbm, "unit": "GB/s",
+    raytrace = {"kernel": "geom_rows_kernel", "bound": "hbm", "achieved": ray_gbs, "peak": hbm, "unit": "GB/s",
                 "frac": ray_gbs / hbm, "algorithmic_bytes_per_launch": ray_bytes,
                 "traffic": measured.get(f"{cfg['name']}:raytrace"),
-                "limiter": "L1/L2 gather latency: the measured DRAM bytes (traffic, one launch of the WFS pupils) "
+                "limiter": "L1 wavefronts of the gathers and issue: the measured DRAM bytes (traffic, one launch of the WFS pupils) "
                            "are a fraction of the algorithmic bytes, each touched screen byte crossing from DRAM "
                            "about once",
                 "note": "algorithmic bytes: one 4-byte screen read per point and layer plus the OPD write"}
@@ -543,7 +543,7 @@ def run_batch(args, bcfg):
         "gpu_launches": int(round(launches_per_step * args.steps)),
         "e2e": {"value": e2e, "unit": "subap-images/s", "h2d_bytes_per_step": h2d // args.steps,
                 "d2h_bytes_per_step": d2h // args.steps},
-        "roofline": {"kernel": "geom_kernel (ray trace of all members)", "bound": "hbm", "achieved": ray_gbs,
+        "roofline": {"kernel": "geom_rows_kernel + geom_kernel (ray trace of all members)", "bound": "hbm", "achieved": ray_gbs,
                      "peak": hbm, "unit": "GB/s", "frac": ray_gbs / hbm, "traffic": None,
                      "peak_source": (f"{src} (MEASURED_PEAKS.json) hbm_gbs" if src == "measured" else "fallback"),
                      "algorithmic_bytes_per_step": ray_bytes},
@@ -756,7 +756,7 @@ def run_science(args, scfg):
     psf_flops = nevl * science_flops(scfg, nX)
     fp32_peak = 148 * 128 * 2 * 1.965e9 / 1e12
     psf_tf = psf_flops / (psf_ms * 1e-3) / 1e12 if psf_ms else 0.0
-    roofline = {"kernel": "geom_kernel (aperture ray trace)", "bound": "hbm", "achieved": ray_gbs, "peak": hbm,
+    roofline = {"kernel": "geom_rows_kernel (aperture ray trace)", "bound": "hbm", "achieved": ray_gbs, "peak": hbm,
                 "unit": "GB/s", "frac": ray_gbs / hbm, "peak_source": src_note + " hbm_gbs", "traffic": None,
                 "algorithmic_bytes_per_launch": ray_bytes,
                 "psf": {"kernels": "evl_psf_rows_kernel + evl_psf_cols_kernel", "achieved": psf_tf,
