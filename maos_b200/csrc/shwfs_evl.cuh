@@ -24,21 +24,31 @@ struct EvlRaster {
 
 // (1) loc_calc_ptt_stride (math/loc.c:653-704) sums over the aperture, per
 // direction: s = {sum a o^2, sum a o, sum a o x, sum a o y}, FP64; grid
-// (ceil(nslot / EVL_SUM_TILES), nevl), 256 threads (one point of a tile
-// each), EVL_SUM_BATCH tiles' loads in flight; sums zeroed before the launch.
+// (ceil(nslot / (nbatch EVL_SUM_BATCH)), nevl), 256 threads (one point of a
+// tile each); a block takes nbatch (evl_sum_batches) times EVL_SUM_BATCH
+// tiles, the loads of a batch in flight together; sums zeroed before the launch.
 // A point's position is its tile's origin plus an offset that is the thread's
 // own, which enters once, at the end: two FP64 fused multiply-adds a point
 // instead of the index arithmetic of its raster position (three directions of
 // 30 m at 1/64 m: 30 -> 24 us, bound by the loads' latency).
-constexpr int EVL_SUM_TILES = 32, EVL_SUM_BATCH = 8;
+constexpr int EVL_SUM_BATCH = 8;
+// Batches per block.  A launch that the chip holds at once (8 blocks of 256
+// threads per SM) is as long as one block, so its blocks take one batch: with
+// four, small apertures' evl_queue calls took 21 -> 25 us (8 m at 1/64 m).
+// Beyond that, fewer blocks mean fewer block sums and atomics: calls of 1600
+// blocks of one, two or four batches' worth took 27.6, 27.1 and 34.6 us, of 11 600
+// 131, 123 and 124, of 52 000 586, 561 and 549.
+__host__ __device__ constexpr int evl_sum_batches(long blocks_of_one, int nsm) {
+	return blocks_of_one <= 8L * nsm ? 1 : blocks_of_one <= 64L * nsm ? 2 : 4;
+}
 __global__ void __launch_bounds__(256) evl_sums_kernel(EvlRaster R, const double* __restrict__ torigx,
-	const double* __restrict__ torigy, const float* __restrict__ opd, double* sums) {
+	const double* __restrict__ torigy, const float* __restrict__ opd, double* sums, int nbatch) {
 	const int e = blockIdx.y, p = threadIdx.x;
 	const float* o = opd + (size_t)e * R.nslot * 256;
 	double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
 #pragma unroll 1
-	for (int b = 0; b < EVL_SUM_TILES; b += EVL_SUM_BATCH) {
-		const int slot0 = blockIdx.x * EVL_SUM_TILES + b;
+	for (int b = 0; b < nbatch; b++) {
+		const int slot0 = (blockIdx.x * nbatch + b) * EVL_SUM_BATCH;
 		float av[EVL_SUM_BATCH], ov[EVL_SUM_BATCH];
 #pragma unroll
 		for (int k = 0; k < EVL_SUM_BATCH; k++) {

@@ -318,9 +318,10 @@ int shwfs_evl_queue(shwfs_ctx* ctx, int isim, int do_psf) {
 	CK(cudaMemsetAsync(E.sums.p, 0, sizeof(double) * 4 * nevl, ctx->stream));
 	{
 		StageMark m(ctx, SHWFS_STAGE_POST);
-		const unsigned nblk = (unsigned)((E.nslot + EVL_SUM_TILES - 1) / EVL_SUM_TILES);
+		const int nb = evl_sum_batches((long)((E.nslot + EVL_SUM_BATCH - 1) / EVL_SUM_BATCH) * nevl, sm_count(ctx));
+		const unsigned nblk = (unsigned)((E.nslot + nb * EVL_SUM_BATCH - 1) / (nb * EVL_SUM_BATCH));
 		evl_sums_kernel<<<dim3(nblk, nevl), 256, 0, ctx->stream>>>(evl_raster(E), E.torigx.p, E.torigy.p, E.opd.p,
-			E.sums.p);
+			E.sums.p, nb);
 		CK(cudaGetLastError());
 	}
 	// (c) PSF sums (psfcomp_r, cuda/sim/perfevl.cu:255-300)
