@@ -243,38 +243,61 @@ int shwfs_evl_psf_reset(shwfs_ctx* ctx) {
 
 }  // extern "C"
 
-// The two-pass transforms serve crops of at most 256 pixels; larger ones keep
-// more outputs than their radix-16 passes form and take the full transforms.
+// Launches of the two-pass transforms (evl_fold_rows_kernel, evl_fold_cols_kernel).
+static unsigned evl_fold_grid(shwfs_ctx* ctx, long lines, int lpb) {
+	return (unsigned)std::min((long)sm_count(ctx) * EVL_FOLD_BLOCKS, (lines + lpb - 1) / lpb);
+}
 template <int N>
-static int evl_launch_fold(shwfs_ctx* ctx, EvlState& E, EvlPsf& P, int nevl) {
+static int evl_fold_rows(shwfs_ctx* ctx, EvlState& E, EvlPsf& P, int nevl) {
 	using F = EvlFold<N>;
 	CK(cudaFuncSetAttribute(evl_fold_rows_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, F::SMEM));
-	CK(cudaFuncSetAttribute(evl_fold_cols_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, F::SMEM));
-	const long most = (long)sm_count(ctx) * EVL_FOLD_BLOCKS;
-	auto grid = [&](long lines) { return (unsigned)std::min(most, (lines + F::LPB - 1) / F::LPB); };
-	evl_fold_rows_kernel<N><<<grid((long)nevl * E.nY), EVL_FOLD_THREADS, F::SMEM, ctx->stream>>>(evl_raster(E), E.opd.p,
-		E.coeff.p, E.pttr, (float)(2.0 / P.wvl), P.offx, P.h, P.tw.p, E.T.p, E.nY, nevl);
+	evl_fold_rows_kernel<N><<<evl_fold_grid(ctx, (long)nevl * E.nY, F::LPB), EVL_FOLD_THREADS, F::SMEM, ctx->stream>>>(
+		evl_raster(E), E.opd.p, E.coeff.p, E.pttr, (float)(2.0 / P.wvl), P.offx, P.h, P.tw.p, E.T.p, E.nY, nevl);
 	CK(cudaGetLastError());
-	evl_fold_cols_kernel<N><<<grid((long)nevl * 2 * P.h), EVL_FOLD_THREADS, F::SMEM, ctx->stream>>>(E.T.p, E.nY, E.nY,
-		P.offy, P.h, P.tw.p, P.psf.p, nevl);
+	return 0;
+}
+template <int N>
+static int evl_fold_cols(shwfs_ctx* ctx, EvlState& E, EvlPsf& P, int nevl) {
+	using F = EvlFold<N>;
+	CK(cudaFuncSetAttribute(evl_fold_cols_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, F::SMEM));
+	evl_fold_cols_kernel<N><<<evl_fold_grid(ctx, (long)nevl * 2 * P.h, F::LPB), EVL_FOLD_THREADS, F::SMEM, ctx->stream>>>(
+		E.T.p, E.nY, E.nY, P.offy, P.h, P.tw.p, P.psf.p, nevl);
 	CK(cudaGetLastError());
 	return 0;
 }
 
+// One wavelength's PSF sums.  Both dimensions write and read the same T, so
+// each is chosen by itself.  Crops of at most 256 pixels from 512 points up can
+// take the two-pass transforms; larger crops keep more outputs than their radix-16
+// passes form and take the full ones.  Rows: always the two passes where they
+// can (a launch of 61 rows of 512 points 2 us shorter, 3891 x 9 of 4096 220).
+// Columns: the two passes only for more lines than a wave of the full
+// transforms holds.  Up to there evl_psf_cols_kernel gives each line a block of its
+// own, 512 threads against the N / 16 of the two passes, and one column is what
+// the launch lasts: 64 columns of 2048 points 2 us shorter than in two passes, 144
+// of 512 1 us, 512 of 2048 1-2 us; equal at 640 of 512 or 768 of 2048; 1280 of
+// 512 2.4 us longer, 2304 of 4096 20 us.  Lines of 4096 fill a block in either
+// form, four blocks of the full one per SM against three, and turn at 256-320.
 template <int N>
 static int evl_launch_psf(shwfs_ctx* ctx, EvlState& E, EvlPsf& P, int nevl) {
-	if constexpr (N >= 512) {
-		if (P.psfsize <= EVL_FOLD_M) return evl_launch_fold<N>(ctx, E, P, nevl);
-	}
 	constexpr int R = 4096 / N;  // rows per block: 512 radix-8 groups, one per thread
 	const size_t smem_r = (size_t)R * evl_row_len<N>() * sizeof(float2), smem_c = (size_t)evl_row_len<N>() * sizeof(float2);
-	if (smem_r > 48 * 1024)
-		CK(cudaFuncSetAttribute(evl_psf_rows_kernel<N, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_r));
-	const EvlRaster Ra = evl_raster(E);
-	const float twoinvwvl = (float)(2.0 / P.wvl);
-	evl_psf_rows_kernel<N, R><<<dim3((E.nY + R - 1) / R, nevl), EVL_THREADS, smem_r, ctx->stream>>>(
-		Ra, E.opd.p, E.coeff.p, E.pttr, twoinvwvl, P.offx, P.h, P.tw.p, E.T.p, E.nY);
-	CK(cudaGetLastError());
+	const bool fold = N >= 512 && P.psfsize <= EVL_FOLD_M;
+	const bool fold_cols = fold && (long)nevl * 2 * P.h > (N == 4096 ? 2L : 4L) * sm_count(ctx);
+	if (fold) {
+		if constexpr (N >= 512) {
+			if (int r = evl_fold_rows<N>(ctx, E, P, nevl)) return r;
+		}
+	} else {
+		if (smem_r > 48 * 1024)
+			CK(cudaFuncSetAttribute(evl_psf_rows_kernel<N, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_r));
+		evl_psf_rows_kernel<N, R><<<dim3((E.nY + R - 1) / R, nevl), EVL_THREADS, smem_r, ctx->stream>>>(
+			evl_raster(E), E.opd.p, E.coeff.p, E.pttr, (float)(2.0 / P.wvl), P.offx, P.h, P.tw.p, E.T.p, E.nY);
+		CK(cudaGetLastError());
+	}
+	if (fold_cols) {
+		if constexpr (N >= 512) return evl_fold_cols<N>(ctx, E, P, nevl);
+	}
 	evl_psf_cols_kernel<N><<<dim3(2 * P.h, nevl), EVL_THREADS, smem_c, ctx->stream>>>(E.T.p, E.nY, E.nY, P.offy, P.h, P.tw.p,
 		P.psf.p);
 	CK(cudaGetLastError());

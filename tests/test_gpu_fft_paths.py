@@ -9,9 +9,11 @@ columns and pupils that do not.  Tolerance: noise-free intensities
 within 1e-5 of the subaperture total, the bar of the other imaging tests.
 
 Science PSF: crops of at most 256 pixels run the two-pass transforms
-(evl_fold_rows_kernel, evl_fold_cols_kernel) for lines of 512 to 4096 points,
-larger crops the full ones; apertures of odd and even width.  Tolerance:
-within 2e-5 of the peak, as the science path's reference test."""
+(evl_fold_rows_kernel) for rows of 512 to 4096 points, larger crops the full
+ones; columns run the two passes (evl_fold_cols_kernel) in launches of more
+lines than the chip holds blocks of the full transforms; apertures of odd and
+even width.  Tolerance: within 2e-5 of the peak, as the science path's
+reference test."""
 import math
 
 import numpy as np
@@ -86,10 +88,11 @@ def test_images_match_plain(N, nopd, pix, lgs):
     ctx.close()
 
 
-@pytest.mark.parametrize("N,ps,nx", [(512, 256, 301), (512, 258, 301), (1024, 50, 1024), (2048, 256, 130), (4096, 16, 701),
-                                     (4096, 256, 700)])
+@pytest.mark.parametrize("N,ps,nx,nevl", [
+    (512, 256, 301, 1), (512, 258, 301, 1), (1024, 50, 1024, 1), (2048, 256, 130, 1), (4096, 16, 701, 1), (4096, 256, 700, 1),
+    (512, 256, 301, 3), (1024, 50, 1024, 12), (2048, 256, 130, 3), (4096, 16, 701, 19), (4096, 256, 700, 2)])
 @pytest.mark.parametrize("pttr", [0, 1])
-def test_cropped_psf_matches_plain(N, ps, nx, pttr):
+def test_cropped_psf_matches_plain(N, ps, nx, nevl, pttr):
     from maos_b200 import shwfs
     rng = np.random.default_rng(N + ps)
     dx, wvl, nxs, sdx = 1 / 32, 1.5e-6, 256, 0.25
@@ -106,12 +109,13 @@ def test_cropped_psf_matches_plain(N, ps, nx, pttr):
     scr = 2e-7 * (np.cos(3 * t)[None] + np.sin(2 * t)[:, None] + np.cos(7 * t[None] + 5 * t[:, None]))
     ctx.atm_set([dict(nx=nxs, ny=nxs, dx=sdx, ox=-nxs / 2 * sdx, oy=-nxs / 2 * sdx, ht=0.0, vx=0.0, vy=0.0, alpha=1.0)], [scr])
     ctx.evl_set_aper(x, y, dx, amp)
-    ctx.evl_add_dir(0.0, 0.0)
+    for _ in range(nevl):
+        ctx.evl_add_dir(0.0, 0.0)
     ctx.evl_set_psf([wvl], [N], [ps], pttr=pttr)
     ctx.evl_queue(0, do_psf=True)
     wfe, coeff = ctx.evl_sync()
-    got, n = ctx.evl_psf(0, 0)
-    assert n == 1
+    got, n = zip(*(ctx.evl_psf(e, 0) for e in range(nevl)))
+    assert set(n) == {1}
     u, v = x / sdx + nxs / 2, y / sdx + nxs / 2
     ju, jv = np.floor(u).astype(int), np.floor(v).astype(int)
     wu, wv = u - ju, v - jv
@@ -128,5 +132,5 @@ def test_cropped_psf_matches_plain(N, ps, nx, pttr):
     f = np.concatenate([np.arange(N - h, N), np.arange(h)])
     F = np.fft.fft(np.fft.fft(E, n=N, axis=0)[f], n=N, axis=1)[:, f]
     ref = np.abs(F) ** 2
-    assert np.abs(got - ref).max() <= 2e-5 * ref.max()
+    assert np.abs(np.stack(got) - ref).max() <= 2e-5 * ref.max()
     ctx.close()
