@@ -500,16 +500,16 @@ __global__ void __launch_bounds__(EVL_FOLD_THREADS, EVL_FOLD_BLOCKS) evl_fold_co
 	evl_fold_lines<N>(s_fold, tw, nline, in, out);
 }
 
-// The PSF sum of one direction (crop column major) as the caller's image, x
-// fastest: out[ax + n ay] = psf[ax n + ay]; blocks of 32 x 8 threads, 32 x 32 tiles.
-__global__ void __launch_bounds__(256) evl_image_kernel(const float* __restrict__ psf, int n, float* __restrict__ out) {
-	__shared__ float s[32][33];
-	const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32, tx = threadIdx.x, ty = threadIdx.y;
-	for (int k = ty; k < 32; k += 8)
-		if (x0 + k < n && y0 + tx < n) s[k][tx] = psf[(size_t)(x0 + k) * n + y0 + tx];
-	__syncthreads();
-	for (int k = ty; k < 32; k += 8)
-		if (y0 + k < n && x0 + tx < n) out[(size_t)(y0 + k) * n + x0 + tx] = s[tx][k];
+// Pixels [i0, i0 + m) of the PSF sum of one direction (crop column major) as
+// the caller's image, x fastest, i = ax + n ay: out[i - i0] = psf[ax n + ay].  out
+// is pinned host memory, so that one launch is the whole read.  The warps' stores are
+// whole 128-byte runs of it, whatever n (32 x 32 tiles through shared memory
+// split them at every row's ends: 258 pixels 57 us a read instead of 48); the loads
+// are a 32-byte sector each, out of L2.
+__global__ void __launch_bounds__(256) evl_image_kernel(const float* __restrict__ psf, int n, int i0, int m,
+	float* __restrict__ out) {
+	const int k = blockIdx.x * 256 + threadIdx.x, i = i0 + k;
+	if (k < m) out[k] = __ldg(psf + (size_t)(i % n) * n + i / n);
 }
 
 // (5) OPD of one direction in aperture order.

@@ -11,6 +11,8 @@ struct EvlPsf {
 	DevBuf<float> psf;   // nevl * psfsize^2 sums, crop column major
 };
 
+constexpr size_t EVL_IMG_MAX = 1 << 20;  // floats of the PSF read's host buffer: 1024 x 1024 pixels, or a part of a larger PSF
+
 struct EvlState {
 	long nloc = 0;
 	double dx = 0, ox = 0, oy = 0;
@@ -32,8 +34,7 @@ struct EvlState {
 	int pttr = 0;
 	long nframe = 0;
 	DevBuf<float2> T;
-	DevBuf<float> img;              // one PSF as an image (shwfs_evl_psf_get), and its pinned copy
-	float* img_h = nullptr;
+	float* img_h = nullptr;         // pinned: a PSF on its way to the caller (shwfs_evl_psf_get)
 	size_t img_h_n = 0;
 	int queued = 0;
 };
@@ -56,7 +57,6 @@ static void evl_free(shwfs_ctx* ctx) {
 		p.tw.free_();
 		p.psf.free_();
 	}
-	E->img.free_();
 	if (E->img_h) cudaFreeHost(E->img_h);
 	if (E->sums_h) cudaFreeHost(E->sums_h);
 	delete E;
@@ -220,6 +220,21 @@ int shwfs_evl_set_psf(shwfs_ctx* ctx, int nwvl, const double* wvl, const int* ne
 			tw[k] = make_float2((float)cos(a), (float)sin(a));
 		}
 		if ((r = dev_upload(ctx, v[w].tw, tw.data(), tw.size()))) return r;
+	}
+	// the buffer that PSFs are read through: made here, since a program reads its
+	// PSFs once, at its end (made in the first read, it cost that read 50-500 us)
+	size_t img = 0;
+	for (auto& p : v) img = std::max(img, std::min((size_t)p.psfsize * p.psfsize, EVL_IMG_MAX));
+	if (E.img_h_n < img) {
+		float* h = nullptr;
+		const cudaError_t e = cudaMallocHost(&h, sizeof(float) * img);
+		if (e != cudaSuccess) {
+			for (auto& p : v) p.tw.free_();
+			return fail(ctx, SHWFS_ENOMEM, "evl_set_psf: cudaMallocHost(%zu bytes): %s", sizeof(float) * img, cudaGetErrorString(e));
+		}
+		if (E.img_h) cudaFreeHost(E.img_h);
+		E.img_h = h;
+		E.img_h_n = img;
 	}
 	for (auto& p : E.psf) {
 		p.tw.free_();
@@ -424,20 +439,13 @@ int shwfs_evl_psf_get(shwfs_ctx* ctx, int ievl, int iwvl, double* psf, long* nfr
 	if (!P.psf.p) {
 		memset(psf, 0, sizeof(double) * nn);
 	} else {
-		if (E.img.n < nn && (r = dev_alloc(ctx, E.img, nn))) return r;
-		if (E.img_h_n < nn) {
-			if (E.img_h) cudaFreeHost(E.img_h);
-			E.img_h = nullptr;
-			E.img_h_n = 0;
-			CK(cudaMallocHost(&E.img_h, sizeof(float) * nn));
-			E.img_h_n = nn;
+		for (size_t i = 0; i < nn; i += E.img_h_n) {
+			const int m = (int)std::min(E.img_h_n, nn - i);
+			evl_image_kernel<<<(m + 255) / 256, 256, 0, ctx->stream>>>(P.psf.p + (size_t)ievl * nn, n, (int)i, m, E.img_h);
+			CK(cudaGetLastError());
+			CK(cudaStreamSynchronize(ctx->stream));
+			f32_to_f64(E.img_h, psf + i, m);
 		}
-		const int nb = (n + 31) / 32;
-		evl_image_kernel<<<dim3(nb, nb), dim3(32, 8), 0, ctx->stream>>>(P.psf.p + (size_t)ievl * nn, n, E.img.p);
-		CK(cudaGetLastError());
-		CK(cudaMemcpyAsync(E.img_h, E.img.p, sizeof(float) * nn, cudaMemcpyDeviceToHost, ctx->stream));
-		CK(cudaStreamSynchronize(ctx->stream));
-		f32_to_f64(E.img_h, psf, nn);
 	}
 	if (nframe) *nframe = ctx->evl->nframe;
 	return 0;

@@ -12,8 +12,8 @@ Science PSF: crops of at most 256 pixels run the two-pass transforms
 (evl_fold_rows_kernel) for rows of 512 to 4096 points, larger crops the full
 ones; columns run the two passes (evl_fold_cols_kernel) in launches of more
 lines than the chip holds blocks of the full transforms; apertures of odd and
-even width.  Tolerance: within 2e-5 of the peak, as the science path's
-reference test."""
+even width; PSFs read whole and in parts.  Tolerance: within 2e-5 of the peak,
+as the science path's reference test."""
 import math
 
 import numpy as np
@@ -89,7 +89,7 @@ def test_images_match_plain(N, nopd, pix, lgs):
 
 
 @pytest.mark.parametrize("N,ps,nx,nevl", [
-    (512, 256, 301, 1), (512, 258, 301, 1), (1024, 50, 1024, 1), (2048, 256, 130, 1), (4096, 16, 701, 1), (4096, 256, 700, 1),
+    (512, 256, 301, 1), (512, 258, 301, 1), (2048, 1100, 301, 1), (1024, 50, 1024, 1), (2048, 256, 130, 1), (4096, 16, 701, 1), (4096, 256, 700, 1),
     (512, 256, 301, 3), (1024, 50, 1024, 12), (2048, 256, 130, 3), (4096, 16, 701, 19), (4096, 256, 700, 2)])
 @pytest.mark.parametrize("pttr", [0, 1])
 def test_cropped_psf_matches_plain(N, ps, nx, nevl, pttr):
@@ -134,3 +134,26 @@ def test_cropped_psf_matches_plain(N, ps, nx, nevl, pttr):
     ref = np.abs(F) ** 2
     assert np.abs(np.stack(got) - ref).max() <= 2e-5 * ref.max()
     ctx.close()
+
+
+def test_first_psf_read_allocates_nothing():
+    import torch
+    from maos_b200 import shwfs
+
+    def exposure(ps):
+        ctx = shwfs.Context(0)
+        x, y = (a.ravel() / 16.0 for a in np.meshgrid(np.arange(64), np.arange(64)))
+        ctx.evl_set_aper(x, y, 1 / 16, np.ones(64 * 64))
+        ctx.evl_add_dir(0.0, 0.0)
+        ctx.evl_set_psf([1e-6], [1024], [ps])
+        ctx.evl_queue(0, do_psf=True)
+        ctx.evl_sync()
+        before = torch.cuda.mem_get_info()[0]
+        ctx.evl_psf(0, 0)
+        return ctx, before, torch.cuda.mem_get_info()[0]
+
+    ctx, _, _ = exposure(16)  # loads the read's kernel
+    ctx.close()
+    ctx, before, after = exposure(1024)
+    ctx.close()
+    assert after == before
