@@ -72,9 +72,7 @@ struct PowfsState {
 	DevBuf<double> mtch_red;          // i0 sum total, max i0 sum (float bits)
 	int tc_ready = 0;
 	std::vector<double> origx_h, origy_h;
-	// sums of x, y and x^2 + y^2 over the pupil points (the focus terms' means):
-	// formed on first use after shwfs_powfs_set_geom
-	bool pt_sums = false;
+	// sums of x, y and x^2 + y^2 over the pupil points (the focus terms' means)
 	double pt_sx = 0, pt_sy = 0, pt_sr = 0;
 	std::vector<DevBuf<int>> gs0_ptr, gs0_col;  // G-tilt operators in CSR, one per amplitude
 	std::vector<DevBuf<float>> gs0_val;
@@ -498,6 +496,25 @@ static WfsState* get_wfs(shwfs_ctx* ctx, int iwfs) {
 	return &ctx->wfs[iwfs];
 }
 
+// The sums over a powfs's nsa nopd^2 pupil points (ox + ix dx, oy + iy dx), ix
+// and iy < n: with i1 = sum i and i2 = sum i^2 over i < n, sum x = n (n sum ox +
+// nsa dx i1) and sum x^2 = n (n sum ox^2 + 2 dx i1 sum ox + nsa dx^2 i2).  The focus
+// terms of every sensor and frame take them from here; summing the 722 k points
+// of the 30 m LGS pupil took 0.7 ms a call.
+static void pupil_sums(PowfsState& p) {
+	const double n = p.d.nopd, dx = p.d.dx, nsa = p.d.nsa, i1 = n * (n - 1) / 2, i2 = i1 * (2 * n - 1) / 3;
+	double sx = 0, sy = 0, sr = 0;
+	for (int isa = 0; isa < p.d.nsa; isa++) {
+		const double x = p.origx_h[isa], y = p.origy_h[isa];
+		sx += x;
+		sy += y;
+		sr += x * x + y * y;
+	}
+	p.pt_sr = n * (n * sr + 2 * dx * i1 * (sx + sy) + 2 * nsa * dx * dx * i2);
+	p.pt_sx = n * (n * sx + nsa * dx * i1);
+	p.pt_sy = n * (n * sy + nsa * dx * i1);
+}
+
 int shwfs_powfs_set_geom(shwfs_ctx* ctx, int ipowfs, const double* origx, const double* origy, const double* amp,
 	int namp, const double* saa) {
 	PowfsState* p = get_powfs(ctx, ipowfs);
@@ -507,7 +524,7 @@ int shwfs_powfs_set_geom(shwfs_ctx* ctx, int ipowfs, const double* origx, const 
 	const int nsa = p->d.nsa, n2 = p->d.nopd * p->d.nopd;
 	p->origx_h.assign(origx, origx + nsa);
 	p->origy_h.assign(origy, origy + nsa);
-	p->pt_sums = false;
+	pupil_sums(*p);
 	if ((r = dev_upload(ctx, p->origx, origx, nsa))) return r;
 	if ((r = dev_upload(ctx, p->origy, origy, nsa))) return r;
 	if ((r = dev_upload_f(ctx, p->amp, amp, (size_t)namp * nsa * n2))) return r;
@@ -810,7 +827,7 @@ int shwfs_wfs_set_opd_terms(shwfs_ctx* ctx, int iwfs, int use_dm, const double* 
 	double focus_llt, const double* lltptt) {
 	WfsState* w = get_wfs(ctx, iwfs);
 	if (!w) return ctx ? fail(ctx, SHWFS_EINVAL, "set_opd_terms: unknown wfs %d", iwfs) : SHWFS_EINVAL;
-	PowfsState& p = ctx->powfs[w->d.ipowfs];
+	const PowfsState& p = ctx->powfs[w->d.ipowfs];
 	if (lltptt && (lltptt[0] != 0 || lltptt[1] != 0) && !p.d.has_llt)
 		return fail(ctx, SHWFS_EINVAL, "set_opd_terms: LLT tip/tilt for WFS %d, whose powfs has no LLT", iwfs);
 	const double t0 = ptt ? ptt[0] : 0, t1 = ptt ? ptt[1] : 0, t2 = ptt ? ptt[2] : 0;
@@ -825,24 +842,7 @@ int shwfs_wfs_set_opd_terms(shwfs_ctx* ctx, int iwfs, int use_dm, const double* 
 	// zoom focus (a, b = the LLT position); expanded about the origin in FP64.
 	double c[4] = {t0, t1, t2, focus_tel + focus_llt};
 	if (focus_tel != 0 || focus_llt != 0) {
-		const int nopd = p.d.nopd;
-		const double n = (double)p.d.nsa * nopd * nopd;
-		if (!p.pt_sums) {
-			double sx = 0, sy = 0, sr = 0;
-			for (int isa = 0; isa < p.d.nsa; isa++)
-				for (int iy = 0; iy < nopd; iy++)
-					for (int ix = 0; ix < nopd; ix++) {
-						const double x = p.origx_h[isa] + ix * p.d.dx, y = p.origy_h[isa] + iy * p.d.dx;
-						sx += x;
-						sy += y;
-						sr += x * x + y * y;
-					}
-			p.pt_sx = sx;
-			p.pt_sy = sy;
-			p.pt_sr = sr;
-			p.pt_sums = true;
-		}
-		// 722 k points of the 30 m LGS pupil: 0.7 ms a call, and a closed loop calls per WFS and frame
+		const double n = (double)p.d.nsa * p.d.nopd * p.d.nopd;
 		const double sx = p.pt_sx, sy = p.pt_sy, sr = p.pt_sr;
 		const double a = p.d.llt_ox, b = p.d.llt_oy;
 		c[0] -= focus_tel * sr / n;
