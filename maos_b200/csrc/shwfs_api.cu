@@ -2029,6 +2029,17 @@ static int frame_powfs(shwfs_ctx* ctx, int ip, const std::vector<int>& wl, int i
 
 // (a) of a physical-optics powfs: one ray-trace launch per batch of pupils
 // (WFS + LLT), and the uplink OTFs of the larger sizes.
+// Long traces (GEOM_LONG gathers per SM: points times layers) have the LLT
+// pupils of the larger sizes beside them, on the aux stream: a handful of blocks in four
+// dependent launches, 35 us for the six LGS at FFT 64.  Shorter traces end with or
+// before that chain, so there is little to run beside, and the fork and join are 2-4 us of
+// the frame: those trace all pupils in one launch and form the OTFs after it.
+// Queued frames, and graph frames, of LGS at FFT 64, one stream -> beside, us:
+// 316 pupils of 32x32 points, 7 layers (2.3 M gathers) 50.7 -> 54.7, 44.7 -> 47.0; 950, 2
+// layers (1.9 M) 65.2 -> 68.7, 58.6 -> 60.8; 600, 7 layers (4.5 M) 57.9 -> 57.9,
+// 56.8 -> 54.2; 4200, 2 layers (8.6 M) 137 -> 134, 136 -> 129; 16 920, 7 layers
+// 473 -> 454, 467 -> 458.
+constexpr long GEOM_LONG = 16384;
 static int trace_powfs(shwfs_ctx* ctx, int ip, const std::vector<int>& wl, int isim) {
 	PowfsState& p = ctx->powfs[ip];
 	int r;
@@ -2047,16 +2058,28 @@ static int trace_powfs(shwfs_ctx* ctx, int ip, const std::vector<int>& wl, int i
 	}
 	const int per = p.d.has_llt ? SHWFS_MAX_ENTRIES / (2 + (p.d.notf == 32 ? nb : 0)) : SHWFS_MAX_ENTRIES;
 	const bool gen_llt = p.d.has_llt && p.d.notf != 32;  // uplink OTFs by the FFT passes
+	auto uplinks = [&](const std::vector<int>& bw, const std::vector<const float*>& lo) {
+		int r = launch_uplink_gen(ctx, p, bw, lo);
+		for (size_t j = 0; j < p.bands.size() && !r; j++) {
+			std::vector<float2*> out;
+			for (int i : bw) out.push_back(ctx->powfs[p.bands[j]].band_lotf[i].p);
+			r = launch_uplink_gen(ctx, ctx->powfs[p.bands[j]], bw, lo, &out);
+		}
+		return r;
+	};
 	for (size_t b = 0; b < wl.size(); b += per) {
 		GeomParams gp, lp;
+		const long gathers = (long)std::min((size_t)per, wl.size() - b) * p.d.nsa * p.d.nopd * p.d.nopd *
+			(long)(ctx->atm.size() + ctx->dm.size());
+		const bool beside = gen_llt && gathers >= GEOM_LONG * sm_count(ctx);
 		geom_init(ctx, gp);
-		if (gen_llt) geom_init(ctx, lp);
+		if (beside) geom_init(ctx, lp);
 		std::vector<int> bw;
 		std::vector<const float*> lo;
 		for (size_t k = b; k < wl.size() && k < b + per; k++) {
 			WfsState& w = ctx->wfs[wl[k]];
 			if ((r = add_wfs_entry(ctx, gp, w, isim, w.opd.p))) return r;
-			if (p.d.has_llt && (r = add_llt_entry(ctx, gen_llt ? lp : gp, w, isim))) return r;
+			if (p.d.has_llt && (r = add_llt_entry(ctx, beside ? lp : gp, w, isim))) return r;
 			if (p.d.has_llt && p.d.notf == 32)
 				for (int ib : p.bands)
 					if ((r = add_llt_band_entry(ctx, gp, w, isim, ctx->powfs[ib], ctx->powfs[ib].band_lotf[wl[k]].p)))
@@ -2064,27 +2087,21 @@ static int trace_powfs(shwfs_ctx* ctx, int ip, const std::vector<int>& wl, int i
 			bw.push_back(wl[k]);
 			lo.push_back(w.lltopd.p);
 		}
-		if (gen_llt) CK(cudaEventRecord(ctx->ev_fork, ctx->stream));
+		if (beside) CK(cudaEventRecord(ctx->ev_fork, ctx->stream));
 		if ((r = launch_geom(ctx, gp))) return r;
-		if (gen_llt) {
-			// the LLT pupils' trace and uplink OTFs (a handful of blocks in four dependent
-			// launches: 35 us for the six LGS at FFT 64) on the aux stream beside the
-			// subapertures' trace, as launch_geom does for the 32-point uplink
+		if (beside) {
 			CK(cudaStreamWaitEvent(ctx->aux, ctx->ev_fork, 0));
 			cudaStream_t main = ctx->stream;
 			ctx->stream = ctx->aux;
 			r = launch_geom_wfs(ctx, lp);
-			if (!r) r = launch_uplink_gen(ctx, p, bw, lo);
-			for (size_t j = 0; j < p.bands.size() && !r; j++) {
-				std::vector<float2*> out;
-				for (int i : bw) out.push_back(ctx->powfs[p.bands[j]].band_lotf[i].p);
-				r = launch_uplink_gen(ctx, ctx->powfs[p.bands[j]], bw, lo, &out);
-			}
+			if (!r) r = uplinks(bw, lo);
 			ctx->stream = main;
 			CK(cudaEventRecord(ctx->ev_join, ctx->aux));
 			CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_join, 0));
-			if (r) return r;
+		} else if (gen_llt) {
+			r = uplinks(bw, lo);
 		}
+		if (r) return r;
 	}
 	return 0;
 }
