@@ -281,7 +281,8 @@ def _roofline(form, cfg, wl, st, units_per_step):
     nlayer = len(cfg["atm"]["ht"])
     ints_bytes, ray_bytes = algorithmic_traffic(cfg, wl.nsa, wl.npix, wl.setup.nopd, wl.setup.notf, nwfs, nlayer)
     ints_ms = st["ints"]["ms_per_launch"]
-    ray_ms = st["raytrace"]["ms_per_step"]  # the WFS pupils, plus any LLT pupils traced in a second launch
+    # the WFS pupils (LLT pupils traced beside them, on the aux stream, are part of the uplink stage, which overlaps this one)
+    ray_ms = st["raytrace"]["ms_per_step"]
     ints_gbs = ints_bytes / (ints_ms * 1e-3) / 1e9 if ints_ms else 0.0
     ray_gbs = ray_bytes / (ray_ms * 1e-3) / 1e9 if ray_ms else 0.0
     measured = {}

@@ -313,7 +313,8 @@ int shwfs_addnoise_dev(shwfs_ctx* ctx, float* ints, long n, const float* bkgrnd2
 /* ---- stage timing: CUDA events around every launch on the context stream,
         as the reference's ctoc instrumentation (cuda/math/common.h:233-267) ---- */
 #define SHWFS_STAGE_RAYTRACE 0 /* (a) ray trace into the subaperture OPD */
-#define SHWFS_STAGE_UPLINK 1   /* LLT ray trace and uplink OTF */
+#define SHWFS_STAGE_UPLINK 1   /* LLT ray trace and uplink OTF; beside the ray trace (a) where they run on a stream
+                                  of their own, so that the stages' sum can exceed the frame */
 #define SHWFS_STAGE_INTS 2     /* (b)-(e) imaging (FFT form: with noise and gradients) */
 #define SHWFS_STAGE_POST 3     /* (d)-(e) noise and gradients after the tensor-core imaging */
 #define SHWFS_NSTAGE 4

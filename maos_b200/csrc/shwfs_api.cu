@@ -878,7 +878,7 @@ int shwfs_wfs_set_opdadd(shwfs_ctx* ctx, int iwfs, const double* opd) {
 
 // ---- frame machinery ----
 
-static int launch_geom_wfs(shwfs_ctx* ctx, GeomParams& gp, bool split = true);
+static int launch_geom_wfs(shwfs_ctx* ctx, GeomParams& gp, bool split = true, int stage = SHWFS_STAGE_RAYTRACE);
 static int sm_count(shwfs_ctx* ctx);
 
 // Appends one pupil to a batched ray-trace launch: per-layer geometry of
@@ -1015,7 +1015,7 @@ static void geom_rows_pick(const GeomParams& gp, int nopd, int nitem, bool small
 // from DRAM once while in L2) and any other pupils in a second launch.  With
 // the screens in L2, the order as listed keeps each block's neighbours on the
 // same footprint, which measured faster.
-static int launch_geom_wfs(shwfs_ctx* ctx, GeomParams& gp, bool split) {
+static int launch_geom_wfs(shwfs_ctx* ctx, GeomParams& gp, bool split, int stage) {
 	if (ctx->trace_order == SHWFS_TRACE_LISTED) gp.interleave = 0;
 	if (split && !gp.interleave && gp.nentry >= 2 && ctx->trace_order != SHWFS_TRACE_LISTED) {
 		double screen = 0;
@@ -1037,8 +1037,8 @@ static int launch_geom_wfs(shwfs_ctx* ctx, GeomParams& gp, bool split) {
 					else rest.e[rest.nentry++] = gp.e[i];
 				}
 				big.interleave = 1;
-				int r = launch_geom_wfs(ctx, big, false);
-				return r ? r : launch_geom_wfs(ctx, rest, false);
+				int r = launch_geom_wfs(ctx, big, false, stage);
+				return r ? r : launch_geom_wfs(ctx, rest, false, stage);
 			}
 		}
 	}
@@ -1059,7 +1059,7 @@ static int launch_geom_wfs(shwfs_ctx* ctx, GeomParams& gp, bool split) {
 				CK(cudaMemsetAsync(gp.e[i].opd, 0, sizeof(float) * gp.e[i].nsa * gp.e[i].nopd * gp.e[i].nopd, ctx->stream));
 	}
 	{
-		StageMark m(ctx, SHWFS_STAGE_RAYTRACE);
+		StageMark m(ctx, stage);
 		const size_t smem = (size_t)gp.nlayer * nopd * 2 * sizeof(int4);
 		if (smem > 160 * 1024) return fail(ctx, SHWFS_EINVAL, "ray trace: %d layers x %d points too large", gp.nlayer, nopd);
 		bool extra = gp.nmirror > 0;
@@ -2093,7 +2093,8 @@ static int trace_powfs(shwfs_ctx* ctx, int ip, const std::vector<int>& wl, int i
 			CK(cudaStreamWaitEvent(ctx->aux, ctx->ev_fork, 0));
 			cudaStream_t main = ctx->stream;
 			ctx->stream = ctx->aux;
-			r = launch_geom_wfs(ctx, lp);
+			// a stage of the aux stream, which the main stream's trace overlaps
+			r = launch_geom_wfs(ctx, lp, true, SHWFS_STAGE_UPLINK);
 			if (!r) r = uplinks(bw, lo);
 			ctx->stream = main;
 			CK(cudaEventRecord(ctx->ev_join, ctx->aux));

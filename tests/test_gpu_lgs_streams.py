@@ -94,3 +94,15 @@ def test_llt_beside_the_trace_equals_one_launch():
     few.close()
     a = a.reshape(len(ISIMS), 2, 2, 2400)[..., :60]  # frame, sensor, axis, subaperture
     assert np.array_equal(a, b.reshape(len(ISIMS), 2, 2, 60))
+
+
+def test_llt_chain_is_booked_as_uplink():
+    """The ray-trace stage times the subapertures' trace alone, also where the LLT pupils are traced beside it."""
+    ctx = _context((2400, 64, 2))
+    _frames(ctx, 0, 2, 2 * 2 * 2400)
+    ctx.profile_enable(True)
+    ctx.profile_read()
+    ctx.frame_queue(3, 0, 2)
+    stages = ctx.profile_read()
+    ctx.close()
+    assert stages["raytrace"][1] == 1 and stages["uplink"][1] == 2
