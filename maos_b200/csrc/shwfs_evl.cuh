@@ -18,7 +18,6 @@ struct EvlRaster {
 	int nslot, ntx, nty, nX, nY;
 	double ox, oy, dx;       // position of raster point (0, 0); spacing
 	const int* tile_slot;    // ntx*nty: slot of a tile, or -1
-	const int* slot_tile;    // nslot: tile of a slot (ty*ntx + tx)
 	const float* amp;        // nslot*256
 };
 

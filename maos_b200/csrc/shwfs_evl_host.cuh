@@ -18,7 +18,7 @@ struct EvlState {
 	double dx = 0, ox = 0, oy = 0;
 	int nX = 0, nY = 0, ntx = 0, nty = 0, nslot = 0;
 	DevBuf<double> torigx, torigy;  // tile origins, by slot
-	DevBuf<int> tile_slot, slot_tile, loc_addr;
+	DevBuf<int> tile_slot, loc_addr;
 	DevBuf<float> amp;              // nslot*256
 	double ipcc = 0, imcc[9] = {0};
 	DevBuf<double> imcc_d;
@@ -45,7 +45,6 @@ static void evl_free(shwfs_ctx* ctx) {
 	E->torigx.free_();
 	E->torigy.free_();
 	E->tile_slot.free_();
-	E->slot_tile.free_();
 	E->loc_addr.free_();
 	E->amp.free_();
 	E->imcc_d.free_();
@@ -74,7 +73,6 @@ static EvlRaster evl_raster(const EvlState& E) {
 	R.oy = E.oy;
 	R.dx = E.dx;
 	R.tile_slot = E.tile_slot.p;
-	R.slot_tile = E.slot_tile.p;
 	R.amp = E.amp.p;
 	return R;
 }
@@ -153,7 +151,6 @@ int shwfs_evl_set_aper(shwfs_ctx* ctx, long nloc, const double* locx, const doub
 	}
 	if ((r = dev_upload(ctx, E.torigx, tox.data(), tox.size())) || (r = dev_upload(ctx, E.torigy, toy.data(), toy.size())) ||
 		(r = dev_upload(ctx, E.tile_slot, tslot.data(), tslot.size())) ||
-		(r = dev_upload(ctx, E.slot_tile, stile.data(), stile.size())) ||
 		(r = dev_upload(ctx, E.loc_addr, addr.data(), addr.size())) ||
 		(r = dev_upload(ctx, E.amp, araster.data(), araster.size())) || (r = dev_upload(ctx, E.imcc_d, imcc, 9)))
 		return r;
