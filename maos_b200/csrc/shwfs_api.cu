@@ -1068,8 +1068,8 @@ static int launch_geom_wfs(shwfs_ctx* ctx, GeomParams& gp, bool split, int stage
 			CK(cudaFuncSetAttribute(geom_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 			CK(cudaFuncSetAttribute(geom_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 		}
-		// GEOM_PTS points per thread with no idle slot where the pupil allows it:
-		// 16x16 pupils 64 threads, 32x32 256, larger ones split over blocks of 256
+		// geom_kernel: GEOM_PTS points per thread with no idle slot where the pupil
+		// allows it, larger pupils split over blocks of 256 threads
 		const int np = nopd * nopd;
 		const int bd = std::min(256, std::max(32, ((np + GEOM_PTS - 1) / GEOM_PTS + 31) / 32 * 32));
 		int bps = (np + GEOM_PTS * bd - 1) / (GEOM_PTS * bd);  // blocks per subaperture

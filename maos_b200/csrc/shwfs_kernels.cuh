@@ -411,7 +411,8 @@ __device__ __forceinline__ float geom_bilerp(float al, float m00, float m10, flo
 
 // EXTRA: the launch has mirror grids, NCPA surfaces or polynomial terms (a
 // closed-loop frame); the open-loop launch compiles without their code.
-// 16x16 and 32x32 pupils run geom_rows_kernel below instead.
+// 16x16 and 32x32 pupils run geom_rows_kernel below instead, unless a screen has 2^30
+// points or more, beyond that kernel's offsets.
 template <bool EXTRA>
 __global__ void __launch_bounds__(256) geom_kernel(const __grid_constant__ GeomParams P, int nopd, int nitem, int bps) {
 	extern __shared__ int4 s_tab[];
@@ -524,10 +525,16 @@ __global__ void __launch_bounds__(256) geom_kernel(const __grid_constant__ GeomP
 // which; a layer with a row that skips a screen row (pupil sampling coarser
 // than the screen) gathers both rows of every point.  One warp covers the two
 // column halves of a 16x16 pupil or the 32 columns of a 32x32 one; the lanes
-// build a layer's line entries together.  The OPD is that of geom_kernel to
-// the bit.  Measured against four gathers a point (7 layers, 6 WFS of 2820
+// build a layer's line entries together.  The layers' and mirrors' sum is that of
+// geom_kernel to the bit (110 launches of 1 to 9000 pupils, 1 to 12 layers, sampled
+// 0.5 to 3 screen cells apart, with and without mirrors); a polynomial's FP64
+// terms are grouped by axis here, so its rounding to FP32 may differ in the
+// last place.  Measured against four gathers a point (7 layers, 6 WFS of 2820
 // pupils): 16x16 63 -> 43 us, with two mirrors and focus 117 -> 55 us; 32x32
 // from 4096^2 screens 201 -> 124 us; three science directions 136 -> 85 us.
+// Sampled coarser than the screen, where every layer takes the four-gather path
+// (1.5 cells, 7 layers, one WFS from 1024^2 screens): 2820 pupils of 16x16 16.5 ->
+// 14.4 us, 9000 33.6 -> 32.8; 800 of 32x32 14.4 -> 14.4, 2820 37.0 -> 34.8.
 // What bounds it now: L1 wavefronts (7.9 M of a 16x16 launch, 28 us) and
 // issue (26 M warp instructions, 24 us) beside each other at 32 warps per SM;
 // 24 or 40 warps per SM (80 or 48 registers a thread) measured 3 % and 60 %
