@@ -99,6 +99,7 @@ def test_lgs_bands_refuse_the_device_input_path():
     opd = torch.zeros(1 << 16, device="cuda:0")
     llt = torch.zeros(1 << 12, device="cuda:0")
     with pytest.raises(shwfs.ShwfsError, match="frame path"):
+        torch.cuda.synchronize()
         ctx.ints_grad_dev(wl.wfs[0], 0, opd, lltopd=llt)
     wl.frame(2)
     assert all(np.isfinite(g).all() for g in wl.frame_sync())

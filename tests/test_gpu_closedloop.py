@@ -76,6 +76,7 @@ def test_closed_loop_frame_matches_reference(ref_lib, cfg_name, isim):
     for k in range(len(wl.wfs)):
         opd_ref, _ = ref_lib.frame_opd(r, k, isim, cfg["dt"])
         opd = torch.zeros(r.nsa * r.nopd ** 2, dtype=torch.float32, device=dev)
+        torch.cuda.synchronize()
         ctx.raytrace_dev(wl.wfs[k], isim, opd)
         ctx.sync()
         o = opd.double().cpu().numpy()
@@ -108,6 +109,7 @@ def test_mirror_points_off_grid_or_nan_add_nothing():
     n = wl.nsa * wl.setup.nopd ** 2
     dev = torch.device("cuda", 0)
     base = torch.zeros(n, dtype=torch.float32, device=dev)
+    torch.cuda.synchronize()
     ctx.raytrace_dev(iw, 2, base)
     grids = [dict(nx=30, ny=30, dx=0.5, ox=-7.5, oy=-7.5, ht=0.0, alpha=-1.0),
              dict(nx=10, ny=10, dx=0.5, ox=40.0, oy=40.0, ht=0.0, alpha=-1.0)]
@@ -115,6 +117,7 @@ def test_mirror_points_off_grid_or_nan_add_nothing():
     for use in (True, False):
         ctx.wfs_set_opd_terms(iw, use_dm=use)
         o = torch.zeros_like(base)
+        torch.cuda.synchronize()
         ctx.raytrace_dev(iw, 2, o)
         ctx.sync()
         assert torch.equal(o, base), use
@@ -122,6 +125,7 @@ def test_mirror_points_off_grid_or_nan_add_nothing():
     ctx.dm_set(grids, [np.full((30, 30), 1e-7), np.ones((10, 10))])
     ctx.wfs_set_opd_terms(iw, use_dm=True)
     o = torch.zeros_like(base)
+    torch.cuda.synchronize()
     ctx.raytrace_dev(iw, 2, o)
     ctx.sync()
     d = (o - base).double().cpu().numpy()

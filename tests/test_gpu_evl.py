@@ -58,6 +58,7 @@ def test_evl_matches_reference(ref_lib, pttr):
         for k, (tx, ty, hs) in enumerate(dirs):
             opd_r, wfe_r, coeff_r, psf_r = e.frame(tx, ty, hs, isim, 1 / 800, pttr=pttr, psfsize=psfsize)
             opd = torch.zeros(nloc, dtype=torch.float32, device="cuda")
+            torch.cuda.synchronize()
             ctx.evl_opd_dev(k, opd)
             ctx.sync()
             o = opd.double().cpu().numpy()

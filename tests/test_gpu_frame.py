@@ -34,6 +34,7 @@ def test_raytrace_matches_reference_prop(ref_lib, isim):
         r.prop_layer(scr, L["dx"], L["ox"], L["oy"], L["ht"], LGS30["thetax"][iw], LGS30["thetay"][iw],
                      LGS30["hs"], -L["vx"] * dt * isim, -L["vy"] * dt * isim, opd=opd_ref)
     opd = torch.zeros(r.nsa * r.nopd ** 2, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
     wl.ctx.raytrace_dev(wl.wfs[iw], isim, opd)
     wl.ctx.sync()
     g = opd.double().cpu().numpy()
@@ -110,12 +111,14 @@ def _noise_statistics(ref_lib, cfg, variant):
     dev = torch.device("cuda", 0)
     o = torch.tensor(opd, dtype=torch.float32, device=dev)
     nf = torch.zeros(r.nsa * r.npix, dtype=torch.float32, device=dev)
+    torch.cuda.synchronize()
     ctx.ints_grad_dev(iw[0], 0, o, None, nf, None, add_noise=False)
     ints = torch.zeros_like(nf)
     s1 = torch.zeros_like(nf, dtype=torch.float64)
     s2 = torch.zeros_like(nf, dtype=torch.float64)
     nframe = 10000
     for k in range(nframe):
+        torch.cuda.synchronize()
         ctx.ints_grad_dev(iw[0], k, o, None, ints, None, add_noise=True)
         d = (ints - nf).double()
         s1 += d

@@ -63,6 +63,7 @@ def test_ztilt_dev_matches_reference(ref_lib):
     iw = wl.wfs[0]
     opd = torch.zeros(r.nsa * r.nopd ** 2, dtype=torch.float32, device="cuda")
     grad = torch.zeros(2 * r.nsa, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
     wl.ctx.raytrace_dev(iw, 11, opd)
     wl.ctx.grad_ztilt_dev(iw, opd, grad)
     wl.ctx.sync()
@@ -78,6 +79,7 @@ def test_gtilt_dev_matches_reference(ref_lib):
     ctx, ip, ws, wl, r = _geom_ctx(ref_lib, NGS8, [(0.0, 0.0)], gradtype=shwfs.SHWFS_GRAD_GTILT)
     opd = torch.zeros(r.nsa * r.nopd ** 2, dtype=torch.float32, device="cuda")
     grad = torch.zeros(2 * r.nsa, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
     ctx.raytrace_dev(ws[0], 17, opd)
     ctx.grad_gtilt_dev(ws[0], opd, grad)
     ctx.sync()

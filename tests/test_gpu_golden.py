@@ -43,6 +43,7 @@ def _run(case, form, variant=None):
         llt = torch.from_numpy(golden(case, "lltopd").ravel().copy()).cuda()
     ints = torch.zeros(nsa * npix, dtype=torch.float32, device="cuda")
     grad = torch.zeros(2 * nsa, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
     wl.ctx.ints_grad_dev(iw, isim, opd, llt, ints, grad)
     wl.ctx.sync()
     ints_ref = golden(case, "ints").ravel(order="F")
@@ -94,6 +95,7 @@ def test_geometric_gradients_match_golden():
     opd = torch.from_numpy(golden("ngs8", "opd").ravel().copy()).cuda()
     gz = torch.zeros(2 * nsa, dtype=torch.float32, device="cuda")
     gg = torch.zeros(2 * nsa, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
     ctx.grad_ztilt_dev(iw, opd, gz)
     ctx.grad_gtilt_dev(iw, opd, gg)
     ctx.sync()
@@ -142,6 +144,7 @@ def test_science_path_matches_golden():
     wfe, coeff = ctx.evl_sync()
     for k in range(ndir):
         opd = torch.zeros(len(x), dtype=torch.float32, device="cuda")
+        torch.cuda.synchronize()
         ctx.evl_opd_dev(k, opd)
         ctx.sync()
         o_ref = golden(f"evl4_dir{k}", "opd").ravel()

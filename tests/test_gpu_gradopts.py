@@ -28,6 +28,7 @@ def _check(ref_lib, cfg, seed=4):
     o = torch.tensor(opd32, dtype=torch.float32, device=dev)
     ints = torch.zeros(ref.nsa * ref.npix, dtype=torch.float32, device=dev)
     g = torch.zeros(2 * ref.nsa, dtype=torch.float32, device=dev)
+    torch.cuda.synchronize()
     ctx.ints_grad_dev(iw[0], 0, o, None, ints, g)
     # the same gradients from the stored intensities (shwfs_grad_dev)
     g2 = torch.zeros(2 * ref.nsa, dtype=torch.float32, device=dev)

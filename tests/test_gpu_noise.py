@@ -26,6 +26,7 @@ def _ctx():
 def _draw(ctx, lam, seed=7, frame=0, **kw):
     import torch
     x = torch.full((N,), float(lam), dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()  # the draws run on the context's own stream
     ctx.addnoise_dev(x, seed=seed, frame=frame, **kw)
     ctx.sync()
     return x.double().cpu().numpy()
@@ -106,6 +107,7 @@ def test_extended_rule_moments():
     dev = "cuda"
     x = torch.tensor(np.tile(x0, reps), dtype=torch.float32, device=dev)
     t = lambda a: torch.tensor(np.tile(a, reps), dtype=torch.float32, device=dev)
+    torch.cuda.synchronize()
     ctx.addnoise_dev(x, seed=11, bkgrnd=bk, bkgrndc=bkc, rne=rne, excess=ex, bkgrnd2=t(b2), bkgrnd2c=t(b2c), qe=t(qe))
     ctx.sync()
     v = x.double().cpu().numpy().reshape(reps, npix)

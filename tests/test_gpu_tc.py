@@ -22,6 +22,7 @@ def _run(ctx, iwfs, nsa, npix, opd, lltopd=None):
     l = torch.tensor(lltopd, dtype=torch.float32, device=dev) if lltopd is not None else None
     ints = torch.zeros(nsa * npix, dtype=torch.float32, device=dev)
     grad = torch.zeros(2 * nsa, dtype=torch.float32, device=dev)
+    torch.cuda.synchronize()
     ctx.ints_grad_dev(iwfs, 0, o, l, ints, grad)
     ctx.sync()
     return ints.double().cpu().numpy(), grad.double().cpu().numpy()

@@ -66,6 +66,7 @@ def test_science_directions_in_either_order():
         ctx.evl_queue(3, do_psf=True)
         wfe, _ = ctx.evl_sync()
         opd = torch.zeros(len(x), dtype=torch.float32, device="cuda")
+        torch.cuda.synchronize()
         ctx.evl_opd_dev(2, opd)
         ctx.sync()
         res.append((np.array(wfe), opd.cpu().numpy(), ctx.evl_psf(1, 0)[0]))

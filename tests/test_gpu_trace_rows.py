@@ -63,6 +63,7 @@ def test_rows_trace_matches_plain(nopd, nsa, step, mirror):
         ref += _plain(ox, oy, nopd, dx, [grid], [surf], False)
         peak += np.abs(surf).max()
     opd = torch.full((nsa * nopd * nopd,), 7.0, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
     ctx.raytrace_dev(iw, 0, opd)
     ctx.sync()
     o = opd.double().cpu().numpy().reshape(ref.shape)
