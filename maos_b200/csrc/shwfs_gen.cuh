@@ -54,8 +54,8 @@ __host__ __device__ constexpr int gen_ls(int n, bool rows) {
 // shared-memory round trip a transform, where radix-2 stages taken two at a
 // time made four with a block barrier each.  52 images of 128 x 128 points, the
 // four passes one after the other with cold caches: 8 + 17 + 18 + 11 -> 8 + 6 +
-// 13 + 8 us; images and gradients in one call 39 -> 19 us (its five launches now
-// set the rate).  ROWS: a line's threads are lanes of one warp.
+// 13 + 8 us; images and gradients in one call 36 -> 15.5 us where calls overlap
+// (its five launches now set the rate), 56 -> 34 back to back on one stream.  ROWS: a line's threads are lanes of one warp.
 // tw[k] = exp(-2 pi i k / N), k < N.
 template <int N, int DIR, bool ROWS>
 __device__ __forceinline__ void gen_fft(float2 (&v)[16], float2* ex, int t, const float2* __restrict__ tw) {
